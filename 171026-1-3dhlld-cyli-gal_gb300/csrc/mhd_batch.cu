@@ -322,9 +322,10 @@ batch_setdt_kernel(const DiscDev *__restrict__ discs, const uint2 *__restrict__ 
     for (int r = local * rows_per_tile; r < (local + 1) * rows_per_tile && r < rows; r++) {
         const int i = 1 + r / nj, j = 1 + r % nj;
         for (int k = 1 + threadIdx.x; k < G.kzmax - 1; k += blockDim.x) {
-            const long long q = cidx(G, i, j, k), nc = G.nc;
-            float v0 = V[q], v1 = V[nc + q], v2v = V[2 * nc + q], v3 = V[3 * nc + q];
-            float v4 = V[4 * nc + q], v5 = V[5 * nc + q], v6 = V[6 * nc + q], v7 = V[7 * nc + q];
+            const long long q = cidx<float>(G, i, j, k);
+            const float *v = V + slot0<float>(q);
+            float v0 = v[0], v1 = v[32], v2v = v[2 * 32], v3 = v[3 * 32];
+            float v4 = v[4 * 32], v5 = v[5 * 32], v6 = v[6 * 32], v7 = v[7 * 32];
             float v2 = v1 * v1 + v2v * v2v + v3 * v3;
             float b2 = v4 * v4 + v5 * v5 + v6 * v6;
             float t1 = sqrtf(v2 + ((float)MHD_GM * v7 + b2) / v0) / G.f.minlength[(long long)i * G.kzmax + k];
@@ -346,7 +347,8 @@ batch_setdt_kernel(const DiscDev *__restrict__ discs, const uint2 *__restrict__ 
         MaxLoc b = sm[0];
         for (int w = 1; w < (int)(blockDim.x >> 5); w++) b = better(b, sm[w]);
         if (b.q >= 0) {
-            const int k = (int)(b.q % G.kzmax), i = (int)(b.q / ((long long)G.kzmax * G.jymax));
+            int i, j, k;
+            cell_of<float>(G, b.q, i, j, k);
             b.v = cfl_rate64_strict<float>(G, V, i, b.q, k);
         }
         D.part[local] = b;
@@ -888,7 +890,7 @@ extern "C" int mhd_batch_upload(mhd_batch *b, int disc, const double *U, const d
     /* all discs share the batch's primitive parity */
     if (b->persistent && b->parity) {
         mhd_ctx *c = b->ctx[disc];
-        BCK(cudaMemcpy(c->Vb, c->Va, 9 * c->nc * sizeof(float), cudaMemcpyDeviceToDevice));
+        BCK(cudaMemcpy(c->Vb, c->Va, 9 * c->ncp * sizeof(float), cudaMemcpyDeviceToDevice));
         c->vcur = 1;
     }
     return MHD_OK;

@@ -7,9 +7,11 @@
  *   SpiralGravity()  -> mhd_spiral_gravity() (spiralgravity.h:20-124)
  *   TVDRK()          -> mhd_tvdrk()          (tvdrungekutta.h:16-78)
  *
- * Device data layout: the reference's own, [m][i][j][k] with k fastest and one
- * ghost cell per side, so host<->device copies are plain memcpy.  The
- * j-independent grid tables (geometric factors, minimum cell length,
+ * Device data layout: in the plain form the reference's own, [m][i][j][k]
+ * with k fastest and one ghost cell per side, so host<->device copies are plain
+ * memcpy; the FP32 forms keep padded rows with the nine variables of 32 cells
+ * together (cidx and slot0 in mhd_dev.cuh), written and read by the FP64
+ * conversion that their transfers make anyway.  The j-independent grid tables (geometric factors, minimum cell length,
  * axisymmetric gravity) are stored once per (i,k).  Compiled with
  * --fmad=false (the gravity probe and the FP64 scalars must round as the
  * reference does).
@@ -197,50 +199,6 @@ static void free_all(mhd_ctx *ctx)
     if (ctx->st_upd) { cudaStreamSynchronize(ctx->st_upd); cudaStreamDestroy(ctx->st_upd); }
     if (ctx->st_aux) { cudaStreamSynchronize(ctx->st_aux); cudaStreamDestroy(ctx->st_aux); }
     if (ctx->st) cudaStreamDestroy(ctx->st);
-    delete ctx->maps;
-}
-
-/* Tensor maps for the TMA-staged update: each FP32 array viewed as a 2D tensor
- * [nvar][nc] (row stride nc * 4 bytes, a multiple of 16 only when nc % 4 == 0;
- * tile coordinates are 32-bit).  cuTensorMapEncodeTiled comes from the driver
- * through the runtime's entry-point query, so the library links no driver
- * library.  NULL when the layout or the driver does not allow it. */
-typedef CUresult (*encode_tiled_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                    const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static UpdMaps *make_upd_maps(mhd_ctx *ctx)
-{
-    if (!ctx->fp32 || ctx->nc % 4 != 0 || ctx->nc + 2 * MHD_UPD_TILE >= (1LL << 31)) return NULL;
-    void *fn = NULL;
-    cudaDriverEntryPointQueryResult qr;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &qr) != cudaSuccess ||
-        qr != cudaDriverEntryPointSuccess || !fn) {
-        cudaGetLastError();
-        return NULL;
-    }
-    encode_tiled_fn enc = (encode_tiled_fn)fn;
-    UpdMaps *m = new (std::nothrow) UpdMaps;
-    if (!m) return NULL;
-    auto mk = [&](CUtensorMap *t, void *base, int nvar, int box) {
-        cuuint64_t dims[2] = {(cuuint64_t)ctx->nc, (cuuint64_t)nvar};
-        cuuint64_t strides[1] = {(cuuint64_t)ctx->nc * sizeof(float)};
-        cuuint32_t boxd[2] = {(cuuint32_t)box, (cuuint32_t)nvar};
-        cuuint32_t es[2] = {1, 1};
-        return enc(t, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, base, dims, strides, boxd, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-    };
-    const int T = MHD_UPD_TILE, W = MHD_UPD_WIDE;
-    bool ok = mk(&m->v[0], ctx->Va, 9, T) && mk(&m->v[1], ctx->Vb, 9, T) && mk(&m->f, ctx->F, 9, T) &&
-              mk(&m->g, ctx->Gf, 9, T) && mk(&m->un, ctx->U, 9, T) && mk(&m->u1, ctx->U1, 9, T) &&
-              mk(&m->fm, ctx->F, 9, W) && mk(&m->gm, ctx->Gf, 9, W) && mk(&m->h, ctx->H, 9, W) &&
-              mk(&m->rho, ctx->rhofloor, 1, T);
-    if (!ok) {
-        delete m;
-        return NULL;
-    }
-    return m;
 }
 
 /* ------------------------------------------------------------------------ */
@@ -381,6 +339,8 @@ extern "C" int mhd_create(const mhd_grid *g, const mhd_params *p, mhd_ctx **out)
 
     Geom &G = ctx->G;
     G.ixmax = ixmax; G.jymax = jymax; G.kzmax = kzmax; G.jy = g->jy; G.irin = g->irin; G.nc = nc;
+    G.kp = ctx->fp32 ? (kzmax + 31) / 32 * 32 : kzmax;
+    G.ncp = ctx->ncp = ctx->fp32 ? 32 + (long long)ixmax * jymax * G.kp : nc;
     double *D = ctx->dtab;
     float *Fd = ctx->ftab;
     G.d.x = D + o_x; G.d.xm = D + o_xm; G.d.oneox = D + o_ox; G.d.oneodx = D + o_odx; G.d.oneodz = D + o_odz;
@@ -408,14 +368,15 @@ extern "C" int mhd_create(const mhd_grid *g, const mhd_params *p, mhd_ctx **out)
     G.repair_irmax = ctx->fp32 ? 4 : 0;
 
     /* ---- state ---- */
-    size_t s9 = 9 * (size_t)nc * ctx->esz;
+    size_t s9 = 9 * (size_t)ctx->ncp * ctx->esz;
     void **bufs9[] = {&ctx->U, &ctx->U1, &ctx->Va, &ctx->Vb, &ctx->Uinit, &ctx->Vinit, &ctx->F, &ctx->Gf, &ctx->H,
                       &ctx->Uraw};
     for (size_t q = 0; q < sizeof bufs9 / sizeof bufs9[0]; q++) {
         CKC(cudaMalloc(bufs9[q], s9));
         CKC(cudaMemsetAsync(*bufs9[q], 0, s9, ctx->st));
     }
-    CKC(cudaMalloc(&ctx->rhofloor, (size_t)nc * ctx->esz));
+    CKC(cudaMalloc(&ctx->rhofloor, (size_t)ctx->ncp * ctx->esz));
+    CKC(cudaMemsetAsync(ctx->rhofloor, 0, (size_t)ctx->ncp * ctx->esz, ctx->st));
     CKC(cudaMalloc(&ctx->Zs, 18 * (size_t)(ixmax - 2) * (jymax - 2) * ctx->esz));
     CKC(cudaMalloc(&ctx->Hb, 9 * (size_t)(ixmax - 2) * (jymax - 2) * ctx->esz));
     if (ctx->pair) {
@@ -443,7 +404,8 @@ extern "C" int mhd_create(const mhd_grid *g, const mhd_params *p, mhd_ctx **out)
     CKC(cudaMallocHost((void **)&ctx->h_part, ctx->npart * sizeof(MaxLoc)));
     CKC(cudaMalloc((void **)&ctx->d_cnt, 3 * 3 * sizeof(int)));
     CKC(cudaMallocHost((void **)&ctx->h_cnt, 3 * 3 * sizeof(int)));
-    ctx->maps = make_upd_maps(ctx);
+    /* the sizes the staged update has always been offered for */
+    ctx->upd_bulk = ctx->fp32 && nc % 4 == 0 && nc + 2 * MHD_UPD_TILE < (1LL << 31);
     ctx->upd_tma = 0;
     ctx->stage_n = 1LL << 24;
     if (ctx->fp32) {
@@ -501,10 +463,12 @@ extern "C" int mhd_current_device(int *ordinal)
 /* ------------------------------------------------------------------------ */
 /* transfers                                                                 */
 /* ------------------------------------------------------------------------ */
-/* host FP64 -> device state of the context's type; with lo (pair-state
- * form) each value is split into the nearest FP32 value and the rest */
-static int put_state(mhd_ctx *ctx, void *dst, const double *src, long long n, float *lo = NULL)
+/* host FP64 array of nvar variables (9, or 1) -> device state array of the
+ * context's type and layout; with lo (pair-state form) each value is split
+ * into the nearest FP32 value and the rest */
+static int put_state(mhd_ctx *ctx, void *dst, const double *src, int nvar, float *lo = NULL)
 {
+    const long long n = nvar * ctx->nc;
     if (!ctx->fp32) {
         CK(cudaMemcpyAsync(dst, src, n * sizeof(double), cudaMemcpyHostToDevice, ctx->st));
         return MHD_OK;
@@ -520,15 +484,17 @@ static int put_state(mhd_ctx *ctx, void *dst, const double *src, long long n, fl
         CK(cudaMemcpyAsync(buf, src + off, m * sizeof(double), cudaMemcpyHostToDevice, ctx->st_cp[b]));
         CK(cudaEventRecord(ctx->ev_cp[b], ctx->st_cp[b]));
         CK(cudaStreamWaitEvent(ctx->st, ctx->ev_cp[b], 0));
-        if (lo) LAUNCH(PK_CVT, launch_cvt_pair(buf, (float *)dst + off, lo + off, m, ctx->st));
-        else LAUNCH(PK_CVT, launch_cvt(buf, (float *)dst + off, m, ctx->st));
+        if (lo) LAUNCH(PK_CVT, launch_cvt_pair(ctx->G, buf, (float *)dst, lo, off, m, ctx->st));
+        else LAUNCH(PK_CVT, launch_cvt(ctx->G, nvar, buf, (float *)dst, off, m, ctx->st));
         CK(cudaEventRecord(ctx->ev_cvt[b], ctx->st));
     }
     return MHD_OK;
 }
 
-static int get_state(mhd_ctx *ctx, double *dst, const void *src, long long n, const float *lo = NULL)
+/* ... and back; nvar = 0: a probe's plain array of n values */
+static int get_state(mhd_ctx *ctx, double *dst, const void *src, int nvar, const float *lo = NULL, long long n = 0)
 {
+    if (nvar) n = nvar * ctx->nc;
     if (!ctx->fp32) {
         CK(cudaMemcpyAsync(dst, src, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
         return MHD_OK;
@@ -540,8 +506,8 @@ static int get_state(mhd_ctx *ctx, double *dst, const void *src, long long n, co
         long long m = n - off < ctx->stage_n ? n - off : ctx->stage_n;
         double *buf = ctx->d_stage + b * ctx->stage_n;
         CK(cudaStreamWaitEvent(ctx->st, ctx->ev_cp[b], 0));      /* the buffer's last copy is done */
-        if (lo) LAUNCH(PK_CVT, launch_cvt_pair_back((const float *)src + off, lo + off, buf, m, ctx->st));
-        else LAUNCH(PK_CVT, launch_cvt_back((const float *)src + off, buf, m, ctx->st));
+        if (lo) LAUNCH(PK_CVT, launch_cvt_pair_back(ctx->G, (const float *)src, lo, buf, off, m, ctx->st));
+        else LAUNCH(PK_CVT, launch_cvt_back(ctx->G, nvar, (const float *)src, buf, off, m, ctx->st));
         CK(cudaEventRecord(ctx->ev_cvt[b], ctx->st));
         CK(cudaStreamWaitEvent(ctx->st_cp[b], ctx->ev_cvt[b], 0));
         CK(cudaMemcpyAsync(dst + off, buf, m * sizeof(double), cudaMemcpyDeviceToHost, ctx->st_cp[b]));
@@ -555,20 +521,19 @@ extern "C" int mhd_upload(mhd_ctx *ctx, const double *U, const double *V, const 
                           const double *rhofloor)
 {
     if (!ctx || !U || !V) return MHD_ERR_ARG;
-    long long n9 = 9 * ctx->nc;
     int rc;
-    if ((rc = put_state(ctx, ctx->U, U, n9, ctx->Ulo))) return rc;
+    if ((rc = put_state(ctx, ctx->U, U, 9, ctx->Ulo))) return rc;
     ctx->vcur = 0;
-    if ((rc = put_state(ctx, ctx->Va, V, n9))) return rc;
-    if ((rc = put_state(ctx, ctx->Uinit, Uinit ? Uinit : U, n9))) return rc;
-    if ((rc = put_state(ctx, ctx->Vinit, Vinit ? Vinit : V, n9))) return rc;
+    if ((rc = put_state(ctx, ctx->Va, V, 9))) return rc;
+    if ((rc = put_state(ctx, ctx->Uinit, Uinit ? Uinit : U, 9))) return rc;
+    if ((rc = put_state(ctx, ctx->Vinit, Vinit ? Vinit : V, 9))) return rc;
     std::vector<double> rf;
     if (!rhofloor) {   /* SaveInitial: rhofloor = U[0]*rhocr (saveinitial.h:40) */
         rf.resize(ctx->nc);
         for (long long q = 0; q < ctx->nc; q++) rf[q] = U[q] * ctx->p.rhocr;
         rhofloor = rf.data();
     }
-    if ((rc = put_state(ctx, ctx->rhofloor, rhofloor, ctx->nc))) return rc;
+    if ((rc = put_state(ctx, ctx->rhofloor, rhofloor, 1))) return rc;
     CK(cudaStreamSynchronize(ctx->st));
     ctx->uploaded = 1;
     return MHD_OK;
@@ -579,10 +544,10 @@ extern "C" int mhd_upload_state(mhd_ctx *ctx, const double *U, const double *V)
     if (!ctx || !U) return MHD_ERR_ARG;
     if (!ctx->uploaded) return MHD_ERR_STATE;
     int rc;
-    if ((rc = put_state(ctx, ctx->U, U, 9 * ctx->nc, ctx->Ulo))) return rc;
+    if ((rc = put_state(ctx, ctx->U, U, 9, ctx->Ulo))) return rc;
     ctx->vcur = 0;
     if (V) {
-        if ((rc = put_state(ctx, ctx->Va, V, 9 * ctx->nc))) return rc;
+        if ((rc = put_state(ctx, ctx->Va, V, 9))) return rc;
     } else if (ctx->pair) {
         LAUNCH(PK_CVT, launch_derive_v_pair(ctx->G, (const float *)ctx->U, ctx->Ulo, (float *)ctx->Va, ctx->st));
     } else if (ctx->fp32) {   /* V = UtoV(U) on the device */
@@ -599,8 +564,8 @@ extern "C" int mhd_download(mhd_ctx *ctx, double *U, double *V)
     if (!ctx) return MHD_ERR_ARG;
     if (!ctx->uploaded) return MHD_ERR_STATE;
     int rc;
-    if (U && (rc = get_state(ctx, U, ctx->U, 9 * ctx->nc, ctx->Ulo))) return rc;
-    if (V && (rc = get_state(ctx, V, vcur_ptr(ctx), 9 * ctx->nc))) return rc;
+    if (U && (rc = get_state(ctx, U, ctx->U, 9, ctx->Ulo))) return rc;
+    if (V && (rc = get_state(ctx, V, vcur_ptr(ctx), 9))) return rc;
     CK(cudaStreamSynchronize(ctx->st));
     return MHD_OK;
 }
@@ -633,9 +598,8 @@ extern "C" int mhd_setdt(mhd_ctx *ctx, double *dt, double *ch, int ijk[3])
     if (ijk) {
         if (best.q < 0) { ijk[0] = ijk[1] = ijk[2] = -1; }
         else {
-            ijk[2] = (int)(best.q % ctx->kzmax);
-            ijk[1] = (int)((best.q / ctx->kzmax) % ctx->jymax);
-            ijk[0] = (int)(best.q / ((long long)ctx->kzmax * ctx->jymax));
+            if (ctx->fp32) cell_of<float>(ctx->G, best.q, ijk[0], ijk[1], ijk[2]);
+            else cell_of<double>(ctx->G, best.q, ijk[0], ijk[1], ijk[2]);
         }
     }
     return MHD_OK;
@@ -791,7 +755,7 @@ static int run_stage(mhd_ctx *ctx, int kind, int last, int *counters)
         if (!hfull) a.Hb = (const T *)ctx->Hb;
         if (int rc = split_fluxes<T>(ctx, V, Vinit, F, Gf, H, hfull)) return rc;
         if (ctx->upd_tma == 1)
-            LAUNCH(PK_UPDATE, launch_update_tma(ctx->G, a, *ctx->maps, ctx->vcur, &ctx->d_sc->err, ctx->st));
+            LAUNCH(PK_UPDATE, launch_update_tma(ctx->G, a, &ctx->d_sc->err, ctx->st));
         else
             LAUNCH(PK_UPDATE, launch_update(ctx->G, a, ctx->st));
     }
@@ -885,8 +849,8 @@ extern "C" int mhd_dbg_limiter(mhd_ctx *ctx, int dir, double dt, double *Vl, dou
         CK(launch_states(dir, ctx->G, (const double *)vcur_ptr(ctx), (const double *)ctx->Vinit, ctx->d_sc,
                          (double *)ctx->F, (double *)ctx->Gf, full_face_box(ctx), ctx->st));
     int rc;
-    if ((rc = get_state(ctx, Vl, ctx->F, nf))) return rc;
-    if ((rc = get_state(ctx, Vr, ctx->Gf, nf))) return rc;
+    if ((rc = get_state(ctx, Vl, ctx->F, 0, NULL, nf))) return rc;
+    if ((rc = get_state(ctx, Vr, ctx->Gf, 0, NULL, nf))) return rc;
     CK(cudaStreamSynchronize(ctx->st));
     return MHD_OK;
 }
@@ -908,7 +872,7 @@ extern "C" int mhd_dbg_flux(mhd_ctx *ctx, int dir, double dt, double ch, double 
     else
         CK(launch_flux(dir, ctx->G, (const double *)vcur_ptr(ctx), (const double *)ctx->Vinit, ctx->d_sc,
                        (double *)ctx->F, full_face_box(ctx), true, ctx->st));
-    int rc = get_state(ctx, Fo, ctx->F, nf);
+    int rc = get_state(ctx, Fo, ctx->F, 0, NULL, nf);
     if (rc) return rc;
     CK(cudaStreamSynchronize(ctx->st));
     return MHD_OK;
@@ -1139,7 +1103,7 @@ extern "C" int mhd_checkpoint_begin(mhd_ctx *ctx, const char *root, int nout, do
         CK(cudaEventCreateWithFlags(&ctx->ev_host, cudaEventDisableTiming | cudaEventBlockingSync));
     }
     /* snapshot on the step stream (ordered after the steps enqueued so far) */
-    if (ctx->fp32) LAUNCH(PK_CVT, launch_cvt_back((const float *)vcur_ptr(ctx), ctx->d_snap, (long long)n, ctx->st));
+    if (ctx->fp32) LAUNCH(PK_CVT, launch_cvt_back(ctx->G, 9, (const float *)vcur_ptr(ctx), ctx->d_snap, 0, (long long)n, ctx->st));
     else CK(cudaMemcpyAsync(ctx->d_snap, vcur_ptr(ctx), n * sizeof(double), cudaMemcpyDeviceToDevice, ctx->st));
     CK(cudaEventRecord(ctx->ev_snap, ctx->st));
     /* device -> host on the I/O stream, beside the following steps */
@@ -1167,24 +1131,26 @@ __global__ void __launch_bounds__(256) diag_kernel(Geom G, const T *__restrict__
 {
     __shared__ double sm[5][8];
     const int nj = G.jymax - 2, rows = (G.ixmax - 2) * nj;
-    const long long nc = G.nc;
+    const long long nc = vstride<T>(G);
     double acc[4] = {0.0, 0.0, 0.0, 0.0}, dmax = 0.0;
     for (int r = blockIdx.x; r < rows; r += gridDim.x) {
         const int i = 1 + r / nj, j = 1 + r % nj;
         const double xi = G.d.x[i], xp = G.d.x[i + 1], xmn = G.d.x[i - 1];
         for (int k = 1 + threadIdx.x; k < G.kzmax - 1; k += blockDim.x) {
-            const long long q = cidx(G, i, j, k);
+            const long long q = cidx<T>(G, i, j, k), b = slot0<T>(q);
             const double dv = G.dvol[(long long)i * G.kzmax + k];
-            double u0 = U[q], u2 = U[2 * nc + q], u7 = U[7 * nc + q], u8 = U[8 * nc + q];
-            if (Ulo) { u0 += Ulo[q]; u2 += Ulo[2 * nc + q]; u7 += Ulo[7 * nc + q]; u8 += Ulo[8 * nc + q]; }
+            double u0 = U[b], u2 = U[2 * nc + b], u7 = U[7 * nc + b], u8 = U[8 * nc + b];
+            if (Ulo) { u0 += Ulo[b]; u2 += Ulo[2 * nc + b]; u7 += Ulo[7 * nc + b]; u8 += Ulo[8 * nc + b]; }
             acc[0] += u0 * dv;
             acc[1] += u2 * dv;
             acc[2] += u7 * dv;
             acc[3] += fabs(u8) * dv;
-            const long long si = (long long)G.jymax * G.kzmax, sj = G.kzmax;
-            double divb = (xp * (double)U[4 * nc + q + si] - xmn * (double)U[4 * nc + q - si]) / (xi * (xp - xmn))
-                          + ((double)U[5 * nc + q + sj] - (double)U[5 * nc + q - sj]) / (xi * 2.0 * G.dy)
-                          + ((double)U[6 * nc + q + 1] - (double)U[6 * nc + q - 1]) / (G.z[k + 1] - G.z[k - 1]);
+            const T *br = U + 4 * nc, *bp = U + 5 * nc, *bz = U + 6 * nc;
+            double divb = (xp * (double)br[nslot<T, 0>(G, q, b, 1)] - xmn * (double)br[nslot<T, 0>(G, q, b, -1)])
+                              / (xi * (xp - xmn))
+                          + ((double)bp[nslot<T, 1>(G, q, b, 1)] - (double)bp[nslot<T, 1>(G, q, b, -1)])
+                              / (xi * 2.0 * G.dy)
+                          + ((double)bz[slot0<T>(q + 1)] - (double)bz[slot0<T>(q - 1)]) / (G.z[k + 1] - G.z[k - 1]);
             dmax = fmax(dmax, fabs(divb));
         }
     }
@@ -1276,7 +1242,7 @@ extern "C" int mhd_set_stage_shape(mhd_ctx *ctx, int fused, int tj, int seg)
 
 extern "C" int mhd_set_update_path(mhd_ctx *ctx, int tma)
 {
-    if (!ctx || tma < 0 || tma > 6 || tma == 3 || tma == 5 || (tma == 1 && !ctx->maps) || (tma > 1 && !ctx->fp32) ||
+    if (!ctx || tma < 0 || tma > 6 || tma == 3 || tma == 5 || (tma == 1 && !ctx->upd_bulk) || (tma > 1 && !ctx->fp32) ||
         (ctx->pair && tma != 0))
         return MHD_ERR_ARG;
     ctx->upd_tma = tma;

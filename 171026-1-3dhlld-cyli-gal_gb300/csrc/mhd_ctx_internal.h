@@ -28,7 +28,7 @@ struct mhd_ctx {
     cudaEvent_t ev_slab[MHD_MAX_SLABS], ev_upd;
     mhd_params p;
     int ix, jy, kz, ixmax, jymax, kzmax, irin;
-    long long nc;
+    long long nc, ncp;           /* cells per variable; slots per variable of the device arrays */
     int fp32;
     size_t esz;
     mhd::Geom G;
@@ -44,11 +44,11 @@ struct mhd_ctx {
     /* stage shape: fused = one kernel for fluxes + update (else the four
      * separate kernels), tile height tj (j) and run length seg (i) */
     int fused, stage_tj, stage_seg;
-    /* tensor maps of the TMA-staged update (precision form, when the layout
-     * allows it; else NULL) and how the split stage's update reads its inputs:
-     * 0 thread loads, 1 TMA-staged tiles, 2 thread loads with an L2 prefetch
-     * of the block one wave ahead */
-    mhd::UpdMaps *maps;
+    /* whether the update staged by bulk copies is offered (precision form),
+     * and how the split stage's update reads its inputs: 0 thread loads, 1
+     * staged tiles, 2 thread loads with an L2 prefetch of the block one wave
+     * ahead */
+    int upd_bulk;
     int upd_tma;
     mhd::StepScalars *d_sc, *h_sc;
     double *d_trig, *h_trig;

@@ -51,9 +51,9 @@ __device__ __forceinline__ void flux_face(const Geom &G, const T *__restrict__ V
 #pragma unroll
         for (int m = 0; m < 9; m++) F[m * nf + q] = Fo[m];
     } else {
-        long long q = cidx(G, i, j, k);
+        T *f = F + slot0<T>(cidx<T>(G, i, j, k));
 #pragma unroll
-        for (int m = 0; m < 9; m++) F[m * G.nc + q] = Fo[m];
+        for (int m = 0; m < 9; m++) f[m * vstride<T>(G)] = Fo[m];
     }
 }
 
@@ -67,9 +67,9 @@ __device__ __forceinline__ void store_face(const Geom &G, T *__restrict__ F, int
 #pragma unroll
         for (int m = 0; m < 9; m++) F[m * nf + q] = Fo[m];
     } else {
-        const long long q = cidx(G, i, j, k);
+        T *f = F + slot0<T>(cidx<T>(G, i, j, k));
 #pragma unroll
-        for (int m = 0; m < 9; m++) F[m * G.nc + q] = Fo[m];
+        for (int m = 0; m < 9; m++) f[m * vstride<T>(G)] = Fo[m];
     }
 }
 
@@ -274,10 +274,10 @@ zwalk_edges_kernel(Geom G, const T *__restrict__ V, const T *__restrict__ Vinit,
                     if (lane == 0) L[m] = m == 3 ? -w2 : w2;
                 }
             } else if (lane == 0) {
-                const long long q0 = cidx(G, i, j, 0);
+                const long long q0 = slot0<T>(cidx<T>(G, i, j, 0));
 #pragma unroll
                 for (int m = 0; m < 9; m++)
-                    L[m] = lim == MHD_LIMITER_MC ? Vinit[(long long)m * G.nc + q0] : Wr[m];
+                    L[m] = lim == MHD_LIMITER_MC ? Vinit[m * vstride<T>(G) + q0] : Wr[m];
             }
             if (lane == 0) {
                 if (lim == MHD_LIMITER_SUPERBEE) {
@@ -325,7 +325,7 @@ zlast_flux_kernel(Geom G, const T *__restrict__ Vinit, const StepScalars *__rest
 #pragma unroll
     for (int m = 0; m < 9; m++) {
         L[m] = Zs[m * nrow + row];
-        if (lim == MHD_LIMITER_MC) R[m] = Vinit[(long long)m * G.nc + cidx(G, i, j, klast + 1)];
+        if (lim == MHD_LIMITER_MC) R[m] = Vinit[m * vstride<T>(G) + slot0<T>(cidx<T>(G, i, j, klast + 1))];
         else if (lim == MHD_LIMITER_SUPERBEE) R[m] = Zs[(9 + m) * nrow + row];
         else R[m] = L[m];
     }
@@ -392,7 +392,7 @@ __device__ __forceinline__ void absorb(const Geom &G, const T *__restrict__ Uini
                                       T u[9])
 {
     const Tabs<T> &tb = tabs<T>(G);
-    long long q = cidx(G, i, j, k);
+    const T *ui0 = Uinit + slot0<T>(cidx<T>(G, i, j, k));
     int ix0 = G.ixmax - 11, kz0 = G.kzmax - 11;
     bool ax = i >= ix0, ac = i <= G.irin, az = zright && k >= kz0;
     if (!(ax || ac || az)) return;
@@ -400,7 +400,7 @@ __device__ __forceinline__ void absorb(const Geom &G, const T *__restrict__ Uini
     T fz = az ? tb.zabs[k - kz0] : T(0);
 #pragma unroll
     for (int m = 0; m < 9; m++) {
-        T ui = Uinit[m * G.nc + q];
+        T ui = ui0[m * vstride<T>(G)];
         T v = u[m];
         if (ax) v -= (fx * (v - ui));
         if (ac) v -= (fc * (v - ui));
@@ -450,7 +450,7 @@ __device__ __forceinline__ void zghost_fill(const Geom &G, const StageArgs<T> &a
         else if (k == 1) kg = G.kzmax - 1;
         else return;
     }
-    const long long nc = G.nc, qg = cidx(G, i, j, kg);
+    const long long nc = vstride<T>(G), qg = cidx<T>(G, i, j, kg), bg = slot0<T>(qg);
     T ug[9], W[9];
 #pragma unroll
     for (int m = 0; m < 9; m++) ug[m] = (flip && m == 3) ? -u[m] : u[m];
@@ -459,7 +459,7 @@ __device__ __forceinline__ void zghost_fill(const Geom &G, const StageArgs<T> &a
     round_stored<T>(G, ug, W);
     T *Uo = (a.kind == 0 || a.kind == 1) ? a.U1 : a.Un;
 #pragma unroll
-    for (int m = 0; m < 9; m++) { Uo[m * nc + qg] = ug[m]; a.Vout[m * nc + qg] = W[m]; }
+    for (int m = 0; m < 9; m++) { Uo[m * nc + bg] = ug[m]; a.Vout[m * nc + bg] = W[m]; }
     if (flags & 1) atomicAdd(&a.counters[0], 1);
     if (flags & 2) atomicAdd(&a.counters[1], 1);
     if (flags & 4) atomicAdd(&a.counters[2], 1);
@@ -469,16 +469,16 @@ __device__ __forceinline__ void zghost_fill(const Geom &G, const StageArgs<T> &a
 template <typename T>
 struct GmemCell {
     const StageArgs<T> &a;
-    long long nc, q;
-    __device__ __forceinline__ T v(int m) const { return a.V[m * nc + q]; }
-    __device__ __forceinline__ T un(int m) const { return a.Un[m * nc + q]; }
-    __device__ __forceinline__ T u1(int m) const { return a.U1[m * nc + q]; }
+    long long nc, q, b;   /* the variables' stride, the cell's slot and its offset */
+    __device__ __forceinline__ T v(int m) const { return a.V[m * nc + b]; }
+    __device__ __forceinline__ T un(int m) const { return a.Un[m * nc + b]; }
+    __device__ __forceinline__ T u1(int m) const { return a.U1[m * nc + b]; }
     __device__ __forceinline__ T rho() const { return a.rhofloor[q]; }
 };
 
 /* kind: 0 U1=U-dtL (Halfstep/FirstStep), 1 U1=(3U+U1-dtL)/4 (SecondStep),
  *       2 U=(U+2(U1-dtL))/3 (ThirdStep), 3 U=(U+U1-dtL)/2 (Fullstep)
- * div[] = the flux divergence of each variable at (i,j,k) (linear index q);
+ * div[] = the flux divergence of each variable at (i,j,k) (slot q);
  * the cell's other inputs come through `in` (global memory, or a tile staged
  * in shared memory). */
 template <typename T, typename In>
@@ -486,7 +486,7 @@ __device__ __forceinline__ int update_core(const Geom &G, const StageArgs<T> &a,
                                            const T div[9], const In &in)
 {
     const StepScalars *sc = a.sc;
-    const long long nc = G.nc;
+    const long long nc = vstride<T>(G), b = slot0<T>(q);
     const T dt = Scal<T>::dt(sc), psicoef = Scal<T>::psi(sc);
     const int kind = a.kind;
     T W[9], S[9], u[9];
@@ -521,7 +521,7 @@ __device__ __forceinline__ int update_core(const Geom &G, const StageArgs<T> &a,
     }
     if (is_bc_source(G, i, j, k)) {
 #pragma unroll
-        for (int m = 0; m < 9; m++) a.Uraw[m * nc + q] = u[m];
+        for (int m = 0; m < 9; m++) a.Uraw[m * nc + b] = u[m];
         if (a.zghost) zghost_fill<T>(G, a, i, j, k, u);
     }
     if (G.scheme == MHD_SCHEME_RK2 && k == 1) u[3] = T(0.0);   /* zboundary.h:87 */
@@ -530,7 +530,7 @@ __device__ __forceinline__ int update_core(const Geom &G, const StageArgs<T> &a,
     round_stored<T>(G, u, W);
     T *Uo = (kind == 0 || kind == 1) ? a.U1 : a.Un;
 #pragma unroll
-    for (int m = 0; m < 9; m++) { Uo[m * nc + q] = u[m]; a.Vout[m * nc + q] = W[m]; }
+    for (int m = 0; m < 9; m++) { Uo[m * nc + b] = u[m]; a.Vout[m * nc + b] = W[m]; }
     return flags;
 }
 
@@ -538,19 +538,19 @@ template <typename T>
 __device__ __forceinline__ int update_apply(const Geom &G, const StageArgs<T> &a, int i, int j, int k,
                                             const T div[9])
 {
-    const long long q = cidx(G, i, j, k);
-    return update_core<T>(G, a, i, j, k, q, div, GmemCell<T>{a, G.nc, q});
+    const long long q = cidx<T>(G, i, j, k);
+    return update_core<T>(G, a, i, j, k, q, div, GmemCell<T>{a, vstride<T>(G), q, slot0<T>(q)});
 }
 
 /* update of one interior cell from the face fluxes in F/G/H */
 template <typename T>
 __device__ __forceinline__ int update_cell(const Geom &G, const StageArgs<T> &a, int i, int j, int k)
 {
-    const long long nc = G.nc, q = cidx(G, i, j, k);
-    const long long si = (long long)G.jymax * G.kzmax, sj = G.kzmax;
+    const long long nc = vstride<T>(G), q = cidx<T>(G, i, j, k), b = slot0<T>(q);
+    const long long bi = nslot<T, 0>(G, q, b, -1), bj = nslot<T, 1>(G, q, b, -1), bk = nslot<T, 2>(G, q, b, -1);
     /* the upper z face of the last cell of a row from the compact Hb, where
      * the split stage keeps it */
-    const T *hu = a.H + q;
+    const T *hu = a.H + b;
     long long hs = nc;
     if (a.Hb && k == G.kzmax - 2) {
         hu = a.Hb + (long long)(i - 1) * (G.jymax - 2) + (j - 1);
@@ -560,8 +560,8 @@ __device__ __forceinline__ int update_cell(const Geom &G, const StageArgs<T> &a,
     geo_factors<T>(G, i, k, g);
 #pragma unroll
     for (int m = 0; m < 9; m++) {
-        const long long mq = m * nc + q;
-        div[m] = flux_div<T>(g, a.F[mq], a.F[mq - si], a.G[mq], a.G[mq - sj], hu[m * hs], a.H[mq - 1]);
+        const long long mn = m * nc;
+        div[m] = flux_div<T>(g, a.F[mn + b], a.F[mn + bi], a.G[mn + b], a.G[mn + bj], hu[m * hs], a.H[mn + bk]);
     }
     return update_apply<T>(G, a, i, j, k, div);
 }
@@ -587,21 +587,23 @@ __device__ __forceinline__ void update_prefetch_ahead(const Geom &G, const Stage
     if (b >= nb) return;
     const int bx = (int)(b % gridDim.x), by = (int)((b / gridDim.x) % gridDim.y), bz = (int)(b / ((long long)gridDim.x * gridDim.y));
     const int k0 = 1 + bx * blockDim.x, i = a.ibeg + bz;
-    const int kn = min((int)blockDim.x, G.kzmax - 1 - k0);
-    const long long nc = G.nc, n9 = 9 * nc;
-    for (int t = lane; t < 7 * (int)blockDim.y * 9; t += 32) {
-        const int arr = t / (9 * blockDim.y), rem = t % (9 * blockDim.y), m = rem / blockDim.y;
-        const int j = 1 + by * blockDim.y + rem % blockDim.y;
-        if (j >= G.jymax - 1 || kn <= 0) continue;
-        const long long q = cidx(G, i, j, k0) + m * nc;
+    if (k0 >= G.kzmax - 1) return;
+    const long long n9 = 9 * G.ncp;
+    /* the rows' cells k0 .. in whole groups of 32 slots: one run per row and array */
+    const int kn = 32 * ((min((int)blockDim.x, G.kzmax - 1 - k0) + 31) / 32);
+    for (int t = lane; t < 7 * (int)blockDim.y; t += 32) {
+        const int arr = t / blockDim.y;
+        const int j = 1 + by * blockDim.y + t % blockDim.y;
+        if (j >= G.jymax - 1) continue;
+        const long long q = cidx<T>(G, i, j, k0), b9 = slot0<T>(q), e9 = b9 + 9 * kn;
         switch (arr) {
-        case 0: prefetch_run<T>(a.V, n9, q, q + kn); break;
-        case 1: prefetch_run<T>(a.F, n9, q, q + kn); break;
-        case 2: prefetch_run<T>(a.G, n9, q, q + kn); break;
-        case 3: prefetch_run<T>(a.H, n9, q - 1, q + kn); break;
-        case 4: prefetch_run<T>(a.Un, n9, q, q + kn); break;
-        case 5: if (a.kind != 0) prefetch_run<T>(a.U1, n9, q, q + kn); break;
-        default: if (m == 0) prefetch_run<T>(a.rhofloor, nc, q, q + kn); break;
+        case 0: prefetch_run<T>(a.V, n9, b9, e9); break;
+        case 1: prefetch_run<T>(a.F, n9, b9, e9); break;
+        case 2: prefetch_run<T>(a.G, n9, b9, e9); break;
+        case 3: prefetch_run<T>(a.H, n9, b9, e9); break;
+        case 4: prefetch_run<T>(a.Un, n9, b9, e9); break;
+        case 5: if (a.kind != 0) prefetch_run<T>(a.U1, n9, b9, e9); break;
+        default: prefetch_run<T>(a.rhofloor, G.ncp, q, q + kn); break;
         }
     }
 }
@@ -626,56 +628,56 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 9 : 1) update_kernel(Geo
 /* ------------------------------------------------------------------------ */
 /* TMA-staged update (precision form)                                        */
 /* ------------------------------------------------------------------------ */
-/* One block per tile of MHD_UPD_TILE consecutive cells of the flat [i][j][k]
- * index.  One thread loads the tile's inputs into shared memory with tensor
- * copies (cp.async.bulk.tensor, completing on an mbarrier): V, F, G, U^n,
- * U^(k), the floor at the tile, and F, G, H at the tile shifted by one plane,
- * one row and one cell (windows MHD_UPD_WIDE wide from the 16-byte boundary at
- * or before the shifted start).  The loads hold no registers, so each SM keeps
- * several tiles (about 40 KB each) in flight; the update itself is
- * update_core, one thread per cell, ghost cells skipped.  The wait is bounded:
+/* One block per tile of MHD_UPD_TILE consecutive slots (four groups of 32).
+ * One thread loads the tile's inputs into shared memory with bulk copies
+ * (cp.async.bulk, completing on an mbarrier): V, F, G, U^n, U^(k) and the
+ * floor at the tile, F one plane and G one row below it, and H from the group
+ * before it -- each one contiguous run in the layout of cidx / slot0.  The
+ * loads hold no registers, so each SM keeps several tiles (about 40 KB each)
+ * in flight; the update itself is update_core, one thread per cell, ghost
+ * cells skipped.  The wait is bounded:
  * a tile whose copies do not land within `spin` polls sets *err, waits as long
  * again for the copies still in flight and leaves the tile untouched.  Should
  * that second wait run out as well, the block exits while bulk copies may
  * still be writing its shared memory -- unsafe, which is one reason this path
  * is an option that stays off, and no test drives either wait to its limit.
- * Measured at 512x512x256: 3.62 ms per launch against 3.38 ms for
- * update_kernel (3.69 ms with all on-chip memory as shared memory): five
+ * Measured at 512x512x256 (with tensor copies of the [m][cells] layout): 3.62
+ * ms per launch against 3.38 ms for update_kernel (3.69 ms with all on-chip
+ * memory as shared memory): five
  * 38 KB tiles per SM keep more bytes in flight than the thread loads, but
- * each block then computes with 4 warps and 20 per SM instead of 32, and the
- * update's arithmetic (sources, the FP64 pressure repair) no longer hides
- * under other warps' loads.  An option (mhd_set_update_path); the thread
- * loads stay the default. */
+ * each block then computes with 4 warps and 20 per SM, and the update's
+ * arithmetic (sources, the FP64 pressure repair) no longer hides under
+ * other warps' loads.  An option (mhd_set_update_path); the thread loads stay
+ * the default. */
 struct UpdTile {
     alignas(128) float v[9 * MHD_UPD_TILE];
     alignas(128) float f[9 * MHD_UPD_TILE];
     alignas(128) float g[9 * MHD_UPD_TILE];
     alignas(128) float un[9 * MHD_UPD_TILE];
     alignas(128) float u1[9 * MHD_UPD_TILE];
-    alignas(128) float fm[9 * MHD_UPD_WIDE];
-    alignas(128) float gm[9 * MHD_UPD_WIDE];
-    alignas(128) float h[9 * MHD_UPD_WIDE];
+    alignas(128) float fm[9 * MHD_UPD_TILE];
+    alignas(128) float gm[9 * MHD_UPD_TILE];
+    alignas(128) float h[9 * (MHD_UPD_TILE + 32)];   /* from the group before the tile */
     alignas(128) float rho[MHD_UPD_TILE];
     alignas(8) unsigned long long bar;
 };
 
-/* a cell's stage inputs from the staged tile (t = the cell's slot) */
+/* a cell's stage inputs from the staged tile (t = the cell's offset in it, slot0 of its slot) */
 struct TileCell {
     const UpdTile &s;
-    int t;
-    __device__ __forceinline__ float v(int m) const { return s.v[m * MHD_UPD_TILE + t]; }
-    __device__ __forceinline__ float un(int m) const { return s.un[m * MHD_UPD_TILE + t]; }
-    __device__ __forceinline__ float u1(int m) const { return s.u1[m * MHD_UPD_TILE + t]; }
+    int t, b;
+    __device__ __forceinline__ float v(int m) const { return s.v[m * 32 + b]; }
+    __device__ __forceinline__ float un(int m) const { return s.un[m * 32 + b]; }
+    __device__ __forceinline__ float u1(int m) const { return s.u1[m * 32 + b]; }
     __device__ __forceinline__ float rho() const { return s.rho[t]; }
 };
 
 __device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 
-__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y, unsigned long long *bar)
+__device__ __forceinline__ void bulk_load(void *dst, const float *src, unsigned bytes, unsigned long long *bar)
 {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-                 " [%0], [%1, {%2, %3}], [%4];"
-                 :: "r"(smem_addr(dst)), "l"((unsigned long long)map), "r"(x), "r"(y), "r"(smem_addr(bar))
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 :: "r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(smem_addr(bar))
                  : "memory");
 }
 
@@ -691,35 +693,32 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long *bar, unsigned 
 
 template <typename T>
 __global__ void __launch_bounds__(MHD_UPD_TILE)
-update_tma_kernel(Geom G, StageArgs<T> a, const __grid_constant__ UpdMaps maps, int vpar, long long qbeg,
-                  int *err, int spin)
+update_tma_kernel(Geom G, StageArgs<T> a, long long qbeg, int *err, int spin)
 {
     static_assert(sizeof(T) == 4, "the staged tile holds FP32 state");
     __shared__ UpdTile s;
     if (a.sc->dtbad) return;
-    const long long q0 = qbeg + (long long)blockIdx.x * MHD_UPD_TILE;
-    const long long si = (long long)G.jymax * G.kzmax, sj = G.kzmax;
-    const int xfm = (int)((q0 - si) & ~3LL), xgm = (int)((q0 - sj) & ~3LL), xh = (int)((q0 - 1) & ~3LL);
-    const int x0 = (int)q0;
+    const long long q0 = qbeg + (long long)blockIdx.x * MHD_UPD_TILE, b0 = slot0<T>(q0);
+    const long long q = q0 + threadIdx.x;
     if (threadIdx.x == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_addr(&s.bar)) : "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        const unsigned narrow = 9 * MHD_UPD_TILE * 4, wide = 9 * MHD_UPD_WIDE * 4;
-        const unsigned bytes = (a.kind != 0 ? 5 : 4) * narrow + 3 * wide + MHD_UPD_TILE * 4;
+        const unsigned tile = 9 * MHD_UPD_TILE * 4, rho = MHD_UPD_TILE * 4;
+        const unsigned bytes = (a.kind != 0 ? 7 : 6) * tile + tile + 9 * 32 * 4 + rho;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
                      :: "r"(smem_addr(&s.bar)), "r"(bytes) : "memory");
-        tma_load_2d(s.v, &maps.v[vpar], x0, 0, &s.bar);
-        tma_load_2d(s.f, &maps.f, x0, 0, &s.bar);
-        tma_load_2d(s.g, &maps.g, x0, 0, &s.bar);
-        tma_load_2d(s.un, &maps.un, x0, 0, &s.bar);
-        if (a.kind != 0) tma_load_2d(s.u1, &maps.u1, x0, 0, &s.bar);
-        tma_load_2d(s.fm, &maps.fm, xfm, 0, &s.bar);
-        tma_load_2d(s.gm, &maps.gm, xgm, 0, &s.bar);
-        tma_load_2d(s.h, &maps.h, xh, 0, &s.bar);
-        tma_load_2d(s.rho, &maps.rho, x0, 0, &s.bar);
+        bulk_load(s.v, a.V + b0, tile, &s.bar);
+        bulk_load(s.f, a.F + b0, tile, &s.bar);
+        bulk_load(s.g, a.G + b0, tile, &s.bar);
+        bulk_load(s.un, a.Un + b0, tile, &s.bar);
+        if (a.kind != 0) bulk_load(s.u1, a.U1 + b0, tile, &s.bar);
+        bulk_load(s.fm, a.F + nslot<T, 0>(G, q0, b0, -1), tile, &s.bar);
+        bulk_load(s.gm, a.G + nslot<T, 1>(G, q0, b0, -1), tile, &s.bar);
+        bulk_load(s.h, a.H + b0 - 9 * 32, tile + 9 * 32 * 4, &s.bar);
+        bulk_load(s.rho, a.rhofloor + q0, rho, &s.bar);
     }
     bool ok = false;
     for (int it = 0; it < spin && !ok; it++) ok = mbar_try_wait(&s.bar, 0);
@@ -728,22 +727,19 @@ update_tma_kernel(Geom G, StageArgs<T> a, const __grid_constant__ UpdMaps maps, 
         for (int it = 0; it < spin && !ok; it++) ok = mbar_try_wait(&s.bar, 0);
         return;
     }
-    const int t = threadIdx.x;
-    const long long q = q0 + t;
-    const int k = (int)(q % G.kzmax);
-    const long long r = q / G.kzmax;
-    const int j = (int)(r % G.jymax), i = (int)(r / G.jymax);
+    const int t = threadIdx.x, b = (int)slot0<T>(t);
+    int i, j, k;
+    cell_of<T>(G, q, i, j, k);
     int flags = 0;
     if (i >= 1 && i <= G.ixmax - 2 && j >= 1 && j <= G.jymax - 2 && k >= 1 && k <= G.kzmax - 2) {
-        const int of = (int)(q - si) - xfm, og = (int)(q - sj) - xgm, oh = (int)(q - 1) - xh;
+        const int hu = b + 9 * 32, hl = (int)slot0<T>(t + 31);
         float gg[6], div[9];
         geo_factors<float>(G, i, k, gg);
 #pragma unroll
         for (int m = 0; m < 9; m++)
-            div[m] = flux_div<float>(gg, s.f[m * MHD_UPD_TILE + t], s.fm[m * MHD_UPD_WIDE + of],
-                                     s.g[m * MHD_UPD_TILE + t], s.gm[m * MHD_UPD_WIDE + og],
-                                     s.h[m * MHD_UPD_WIDE + oh + 1], s.h[m * MHD_UPD_WIDE + oh]);
-        flags = update_core<float>(G, a, i, j, k, q, div, TileCell{s, t});
+            div[m] = flux_div<float>(gg, s.f[m * 32 + b], s.fm[m * 32 + b], s.g[m * 32 + b], s.gm[m * 32 + b],
+                                     s.h[m * 32 + hu], s.h[m * 32 + hl]);
+        flags = update_core<float>(G, a, i, j, k, q, div, TileCell{s, t, b});
     }
     add_counters(flags, a.counters);
 }
@@ -806,7 +802,7 @@ __global__ void __launch_bounds__(128, 8) zupdate_kernel(Geom G, StageArgs<T> a)
         }
     }
     __syncwarp();
-    const long long nc = G.nc, si = (long long)G.jymax * G.kzmax, sj = G.kzmax;
+    const long long nc = vstride<T>(G);
     unsigned c0 = 0, c1 = 0, c2 = 0;
     for (int rr = 0; rr < ROWS; rr++) {
         const long long r = row0 + rr;
@@ -833,13 +829,14 @@ __global__ void __launch_bounds__(128, 8) zupdate_kernel(Geom G, StageArgs<T> a)
             }
             __syncwarp();
             if (live) {
-                const long long q = cidx(G, i, j, k);
+                const long long q = cidx<T>(G, i, j, k), b = slot0<T>(q);
+                const long long bi = nslot<T, 0>(G, q, b, -1), bj = nslot<T, 1>(G, q, b, -1);
                 T g[6], div[9];
                 geo_factors<T>(G, i, k, g);
 #pragma unroll
                 for (int m = 0; m < 9; m++) {
-                    const long long mq = m * nc + q;
-                    div[m] = flux_div<T>(g, a.F[mq], a.F[mq - si], a.G[mq], a.G[mq - sj], sh[w][m][lane + 1],
+                    const long long mn = m * nc;
+                    div[m] = flux_div<T>(g, a.F[mn + b], a.F[mn + bi], a.G[mn + b], a.G[mn + bj], sh[w][m][lane + 1],
                                          sh[w][m][lane]);
                 }
                 int flags = update_apply<T>(G, a, i, j, k, div);
@@ -905,7 +902,7 @@ __global__ void __launch_bounds__(32 * (TJ + 1), MINB) stage_kernel(Geom G, Stag
     const T *__restrict__ V = a.V;
     const T *__restrict__ Vinit = a.Vinit;
     const StepScalars *__restrict__ sc = a.sc;
-    const long long nc = G.nc, nall = 9 * nc, si = (long long)G.jymax * G.kzmax;
+    const long long nc = vstride<T>(G), nall = 9 * G.ncp;
     unsigned c0 = 0, c1 = 0, c2 = 0;
     T f[9];
     if (live) {
@@ -929,26 +926,28 @@ __global__ void __launch_bounds__(32 * (TJ + 1), MINB) stage_kernel(Geom G, Stag
             }
         } else {
             /* next plane's cold inputs: U^n, U^(k), rhofloor rows of the
-             * tile, and the V plane the r reconstruction reaches next */
+             * tile, and the V plane the r reconstruction reaches next.  A
+             * row's 32 cells are one run over all variables in the FP32
+             * forms' layout, one run per variable in the plain form's. */
+            constexpr int NV = sizeof(T) == 4 ? 1 : 9, RUN = sizeof(T) == 4 ? 9 * 32 : 32;
             if (i + 1 < ib) {
-                const long long row0 = ((long long)(i + 1) * G.jymax + j0) * G.kzmax + k0;
-                for (int t = lane; t < 19 * TJ; t += 32) {
+                for (int t = lane; t < (2 * NV + 1) * TJ; t += 32) {
                     const int v = t / TJ, r = t - v * TJ;
                     if (j0 + r >= G.jymax - 1) continue;
-                    const long long e0 = row0 + (long long)r * G.kzmax;
-                    if (v < 9) prefetch_run<T>(a.Un, nall, v * nc + e0, v * nc + e0 + 32);
-                    else if (v < 18) { if (a.kind != 0) prefetch_run<T>(a.U1, nall, (v - 9) * nc + e0, (v - 9) * nc + e0 + 32); }
-                    else prefetch_run<T>(a.rhofloor, nc, e0, e0 + 32);
+                    const long long q = cidx<T>(G, i + 1, j0 + r, k0), e0 = slot0<T>(q);
+                    if (v < NV) prefetch_run<T>(a.Un, nall, v * nc + e0, v * nc + e0 + RUN);
+                    else if (v < 2 * NV) {
+                        if (a.kind != 0) prefetch_run<T>(a.U1, nall, (v - NV) * nc + e0, (v - NV) * nc + e0 + RUN);
+                    } else prefetch_run<T>(a.rhofloor, G.ncp, q, q + 32);
                 }
             }
             if (i + 3 < G.ixmax) {
-                const long long pl0 = (long long)(i + 3) * si;
-                for (int t = lane; t < 9 * (TJ + 4); t += 32) {
+                for (int t = lane; t < NV * (TJ + 4); t += 32) {
                     const int v = t / (TJ + 4), jr = j0 - 2 + (t - v * (TJ + 4));
                     if (jr < 0 || jr >= G.jymax) continue;
-                    const long long e0 = v * nc + pl0 + (long long)jr * G.kzmax;
-                    const int ka = max(k0 - 2, 0), kb = min(k0 + 34, G.kzmax);
-                    prefetch_run<T>(V, nall, e0 + ka, e0 + kb);
+                    const long long e0 = v * nc + slot0<T>(cidx<T>(G, i + 3, jr, k0));
+                    if (sizeof(T) == 4) prefetch_run<T>(V, nall, e0, e0 + RUN);
+                    else prefetch_run<T>(V, nall, e0 - min(k0, 2), e0 + min(34, G.kzmax - k0));
                 }
             }
             if (kin && j0 < G.jymax - 1) {
@@ -1061,11 +1060,12 @@ __device__ __forceinline__ int ghost_cell(const Geom &G, const StageArgs<T> &a, 
     int si, sj, sk;
     unsigned neg;
     ghost_source(G, i, j, k, si, sj, sk, neg);
-    const long long nc = G.nc, q = cidx(G, i, j, k), qs = cidx(G, si, sj, sk);
+    const long long nc = vstride<T>(G), q = cidx<T>(G, i, j, k), b = slot0<T>(q);
+    const long long bs = slot0<T>(cidx<T>(G, si, sj, sk));
     T u[9], W[9];
 #pragma unroll
     for (int m = 0; m < 9; m++) {
-        T v = a.Uraw[m * nc + qs];
+        T v = a.Uraw[m * nc + bs];
         u[m] = ((neg >> m) & 1u) ? -v : v;
     }
     if (G.scheme == MHD_SCHEME_RK2 && k == 1) u[3] = T(0.0);
@@ -1074,7 +1074,7 @@ __device__ __forceinline__ int ghost_cell(const Geom &G, const StageArgs<T> &a, 
     round_stored<T>(G, u, W);
     T *Uo = (a.kind == 0 || a.kind == 1) ? a.U1 : a.Un;
 #pragma unroll
-    for (int m = 0; m < 9; m++) { Uo[m * nc + q] = u[m]; a.Vout[m * nc + q] = W[m]; }
+    for (int m = 0; m < 9; m++) { Uo[m * nc + b] = u[m]; a.Vout[m * nc + b] = W[m]; }
     return flags;
 }
 
@@ -1105,9 +1105,10 @@ __device__ __forceinline__ MaxLoc better(MaxLoc a, MaxLoc b)
 template <typename T>
 __device__ __forceinline__ double cfl_rate64(const Geom &G, const T *__restrict__ V, int i, long long q, int k)
 {
-    const long long nc = G.nc;
-    double v0 = V[q], v1 = V[nc + q], v2v = V[2 * nc + q], v3 = V[3 * nc + q];
-    double v4 = V[4 * nc + q], v5 = V[5 * nc + q], v6 = V[6 * nc + q], v7 = V[7 * nc + q];
+    const long long nc = vstride<T>(G);
+    const T *v = V + slot0<T>(q);
+    double v0 = v[0], v1 = v[nc], v2v = v[2 * nc], v3 = v[3 * nc];
+    double v4 = v[4 * nc], v5 = v[5 * nc], v6 = v[6 * nc], v7 = v[7 * nc];
     double v2 = v1 * v1 + v2v * v2v + v3 * v3;
     double b2 = v4 * v4 + v5 * v5 + v6 * v6;
     double t1 = sqrt(v2 + (MHD_GM * v7 + b2) / v0) / G.minlength[(long long)i * G.kzmax + k];
@@ -1125,9 +1126,10 @@ template <typename T>
 __device__ __forceinline__ double cfl_rate64_strict(const Geom &G, const T *__restrict__ V, int i, long long q,
                                                     int k)
 {
-    const long long nc = G.nc;
-    double v0 = V[q], v1 = V[nc + q], v2v = V[2 * nc + q], v3 = V[3 * nc + q];
-    double v4 = V[4 * nc + q], v5 = V[5 * nc + q], v6 = V[6 * nc + q], v7 = V[7 * nc + q];
+    const long long nc = vstride<T>(G);
+    const T *v = V + slot0<T>(q);
+    double v0 = v[0], v1 = v[nc], v2v = v[2 * nc], v3 = v[3 * nc];
+    double v4 = v[4 * nc], v5 = v[5 * nc], v6 = v[6 * nc], v7 = v[7 * nc];
     double v2 = v1 * v1 + v2v * v2v + v3 * v3;
     double b2 = v4 * v4 + v5 * v5 + v6 * v6;
     double t1 = sqrt(v2 + (MHD_GM * v7 + b2) / v0) / G.minlength[(long long)i * G.kzmax + k];
@@ -1152,14 +1154,15 @@ setdt_kernel(Geom G, const T *__restrict__ V, MaxLoc *part)
     for (int r = blockIdx.x; r < rows; r += gridDim.x) {
         const int i = 1 + r / nj, j = 1 + r % nj;
         for (int k = 1 + threadIdx.x; k < G.kzmax - 1; k += blockDim.x) {
-            const long long q = cidx(G, i, j, k);
+            const long long q = cidx<T>(G, i, j, k);
             double tmp;
             if (sizeof(T) == 8) {
                 tmp = cfl_rate64<T>(G, V, i, q, k);
             } else {
-                const long long nc = G.nc;
-                float v0 = V[q], v1 = V[nc + q], v2v = V[2 * nc + q], v3 = V[3 * nc + q];
-                float v4 = V[4 * nc + q], v5 = V[5 * nc + q], v6 = V[6 * nc + q], v7 = V[7 * nc + q];
+                const long long nc = vstride<T>(G);
+                const T *v = V + slot0<T>(q);
+                float v0 = v[0], v1 = v[nc], v2v = v[2 * nc], v3 = v[3 * nc];
+                float v4 = v[4 * nc], v5 = v[5 * nc], v6 = v[6 * nc], v7 = v[7 * nc];
                 float v2 = v1 * v1 + v2v * v2v + v3 * v3;
                 float b2 = v4 * v4 + v5 * v5 + v6 * v6;
                 float t1 = sqrtf(v2 + ((float)MHD_GM * v7 + b2) / v0) / (float)G.f.minlength[(long long)i * G.kzmax + k];
@@ -1183,7 +1186,8 @@ setdt_kernel(Geom G, const T *__restrict__ V, MaxLoc *part)
         MaxLoc b = sm[0];
         for (int w = 1; w < (int)(blockDim.x >> 5); w++) b = better(b, sm[w]);
         if (sizeof(T) == 4 && b.q >= 0) {
-            const int k = (int)(b.q % G.kzmax), i = (int)(b.q / ((long long)G.kzmax * G.jymax));
+            int i, j, k;
+            cell_of<T>(G, b.q, i, j, k);
             b.v = cfl_rate64_strict<T>(G, V, i, b.q, k);
         }
         part[blockIdx.x] = b;
@@ -1193,15 +1197,45 @@ setdt_kernel(Geom G, const T *__restrict__ V, MaxLoc *part)
 /* ------------------------------------------------------------------------ */
 /* conversions                                                               */
 /* ------------------------------------------------------------------------ */
-template <typename T>
-__global__ void cvt_from_f64(const double *__restrict__ src, T *__restrict__ dst, long long n)
+/* Values off .. off+n-1 of a host array [nvar][i][j][k] (FP64, in src / dst from
+ * its first) into or out of a state array: f(host index from off, device
+ * offset) handles one value.  Index type I: 32 bits where the array allows it,
+ * for its cheap division. */
+template <typename T, typename I, typename F>
+__device__ __forceinline__ void each_value_i(const Geom &G, int nvar, long long off, long long n, F f)
 {
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
-        dst[t] = (T)src[t];
+    const I kz = (I)G.kzmax, nrow = (I)((long long)G.ixmax * G.jymax);
+    const long long q0 = cidx<T>(G, 0, 0, 0), row = sstride<T>(G, 1);
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+        const I h = (I)(off + t), r = h / kz, m = r / nrow;
+        const long long q = q0 + (long long)(r - m * nrow) * row + (long long)(h - r * kz);
+        f(t, nvar == 1 ? q : (long long)m * vstride<T>(G) + slot0<T>(q));
+    }
+}
+template <typename T, typename F>
+__device__ __forceinline__ void each_value(const Geom &G, int nvar, long long off, long long n, F f)
+{
+    if (nvar * G.nc < (1LL << 32)) each_value_i<T, unsigned>(G, nvar, off, n, f);
+    else each_value_i<T, unsigned long long>(G, nvar, off, n, f);
 }
 
 template <typename T>
-__global__ void cvt_to_f64(const T *__restrict__ src, double *__restrict__ dst, long long n)
+__global__ void cvt_from_f64(Geom G, int nvar, const double *__restrict__ src, T *__restrict__ dst, long long off,
+                             long long n)
+{
+    each_value<T>(G, nvar, off, n, [&](long long h, long long d) { dst[d] = (T)src[h]; });
+}
+
+template <typename T>
+__global__ void cvt_to_f64(Geom G, int nvar, const T *__restrict__ src, double *__restrict__ dst, long long off,
+                           long long n)
+{
+    each_value<T>(G, nvar, off, n, [&](long long h, long long d) { dst[h] = (double)src[d]; });
+}
+
+/* a probe's plain array (no state layout) to FP64 */
+template <typename T>
+__global__ void cvt_linear_to_f64(const T *__restrict__ src, double *__restrict__ dst, long long n)
 {
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
         dst[t] = (double)src[t];
@@ -1212,15 +1246,18 @@ __global__ void cvt_to_f64(const T *__restrict__ src, double *__restrict__ dst, 
 template <typename T>
 __global__ void __launch_bounds__(256) derive_v_kernel(Geom G, const T *__restrict__ U, T *__restrict__ V)
 {
-    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < G.nc;
-         q += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(q / ((long long)G.jymax * G.kzmax));
+    const long long nc = vstride<T>(G);
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < G.nc;
+         t += (long long)gridDim.x * blockDim.x) {
+        const long long r = t / G.kzmax;
+        const int i = (int)(r / G.jymax);
+        const long long b = slot0<T>(cidx<T>(G, i, (int)(r % G.jymax), (int)(t % G.kzmax)));
         T u[9], w[9];
 #pragma unroll
-        for (int m = 0; m < 9; m++) u[m] = U[m * G.nc + q];
+        for (int m = 0; m < 9; m++) u[m] = U[m * nc + b];
         utov<T>(G, i, u, w);
 #pragma unroll
-        for (int m = 0; m < 9; m++) V[m * G.nc + q] = w[m];
+        for (int m = 0; m < 9; m++) V[m * nc + b] = w[m];
     }
 }
 
@@ -1238,7 +1275,7 @@ __global__ void source_kernel(Geom G, const T *__restrict__ V, const StepScalars
     int i = (int)(r / G.jymax);
     T W[9], Sv[9];
 #pragma unroll
-    for (int m = 0; m < 9; m++) W[m] = V[m * G.nc + tid];
+    for (int m = 0; m < 9; m++) W[m] = V[m * vstride<T>(G) + slot0<T>(cidx<T>(G, i, j, k))];
     source_at<T>(G, *sc, trig, trigf, i, j, k, W, Sv);
 #pragma unroll
     for (int m = 0; m < 9; m++) S[m * G.nc + tid] = (double)Sv[m];
@@ -1400,16 +1437,14 @@ cudaError_t launch_update_t(const Geom &G, const StageArgs<T> &a, cudaStream_t s
 
 /* the TMA-staged update over the tiles that cover the interior planes */
 template <typename T>
-cudaError_t launch_update_tma_t(const Geom &G, const StageArgs<T> &a, const UpdMaps &maps, int vpar, int *err,
-                                cudaStream_t st)
+cudaError_t launch_update_tma_t(const Geom &G, const StageArgs<T> &a, int *err, cudaStream_t st)
 {
     if constexpr (sizeof(T) != 4) {
         return cudaErrorNotSupported;
     } else {
-        const long long si = (long long)G.jymax * G.kzmax;
-        const long long qbeg = si & ~3LL, qend = (long long)(G.ixmax - 1) * si;
+        const long long qbeg = cidx<T>(G, 1, 0, 1), qend = cidx<T>(G, G.ixmax - 1, 0, 1);
         const long long nt = (qend - qbeg + MHD_UPD_TILE - 1) / MHD_UPD_TILE;
-        update_tma_kernel<T><<<(unsigned)nt, MHD_UPD_TILE, 0, st>>>(G, a, maps, vpar, qbeg, err, 1 << 20);
+        update_tma_kernel<T><<<(unsigned)nt, MHD_UPD_TILE, 0, st>>>(G, a, qbeg, err, 1 << 20);
         return cudaGetLastError();
     }
 }
@@ -1480,9 +1515,10 @@ cudaError_t launch_source_t(const Geom &G, const T *V, const StepScalars *sc, co
 }
 
 template <typename T>
-cudaError_t launch_cvt_t(const double *src, T *dst, long long n, cudaStream_t st)
+cudaError_t launch_cvt_t(const Geom &G, int nvar, const double *src, T *dst, long long off, long long n,
+                         cudaStream_t st)
 {
-    cvt_from_f64<T><<<1024, 256, 0, st>>>(src, dst, n);
+    cvt_from_f64<T><<<1024, 256, 0, st>>>(G, nvar, src, dst, off, n);
     return cudaGetLastError();
 }
 
@@ -1494,9 +1530,11 @@ cudaError_t launch_derive_v_t(const Geom &G, const T *U, T *V, cudaStream_t st)
 }
 
 template <typename T>
-cudaError_t launch_cvt_back_t(const T *src, double *dst, long long n, cudaStream_t st)
+cudaError_t launch_cvt_back_t(const Geom &G, int nvar, const T *src, double *dst, long long off, long long n,
+                              cudaStream_t st)
 {
-    cvt_to_f64<T><<<1024, 256, 0, st>>>(src, dst, n);
+    if (nvar == 0) cvt_linear_to_f64<T><<<1024, 256, 0, st>>>(src + off, dst, n);
+    else cvt_to_f64<T><<<1024, 256, 0, st>>>(G, nvar, src, dst, off, n);
     return cudaGetLastError();
 }
 
@@ -1539,10 +1577,9 @@ cudaError_t launch_cvt_back_t(const T *src, double *dst, long long n, cudaStream
     {                                                                                                        \
         return launch_update_t<T>(G, a, st);                                                                 \
     }                                                                                                        \
-    cudaError_t launch_update_tma(const Geom &G, const StageArgs<T> &a, const UpdMaps &maps, int vpar,      \
-                                  int *err, cudaStream_t st)                                                 \
+    cudaError_t launch_update_tma(const Geom &G, const StageArgs<T> &a, int *err, cudaStream_t st)           \
     {                                                                                                        \
-        return launch_update_tma_t<T>(G, a, maps, vpar, err, st);                                            \
+        return launch_update_tma_t<T>(G, a, err, st);                                                        \
     }                                                                                                        \
     cudaError_t launch_ghost(const Geom &G, const StageArgs<T> &a, cudaStream_t st)                           \
     {                                                                                                        \
@@ -1569,13 +1606,15 @@ cudaError_t launch_cvt_back_t(const T *src, double *dst, long long n, cudaStream
     {                                                                                                        \
         return launch_source_t<T>(G, V, sc, trig, trigf, S, st);                                             \
     }                                                                                                        \
-    cudaError_t launch_cvt(const double *src, T *dst, long long n, cudaStream_t st)                          \
+    cudaError_t launch_cvt(const Geom &G, int nvar, const double *src, T *dst, long long off, long long n,   \
+                           cudaStream_t st)                                                                  \
     {                                                                                                        \
-        return launch_cvt_t<T>(src, dst, n, st);                                                             \
+        return launch_cvt_t<T>(G, nvar, src, dst, off, n, st);                                               \
     }                                                                                                        \
-    cudaError_t launch_cvt_back(const T *src, double *dst, long long n, cudaStream_t st)                     \
+    cudaError_t launch_cvt_back(const Geom &G, int nvar, const T *src, double *dst, long long off,           \
+                                long long n, cudaStream_t st)                                                \
     {                                                                                                        \
-        return launch_cvt_back_t<T>(src, dst, n, st);                                                        \
+        return launch_cvt_back_t<T>(G, nvar, src, dst, off, n, st);                                          \
     }                                                                                                        \
     cudaError_t launch_derive_v(const Geom &G, const T *U, T *V, cudaStream_t st)                           \
     {                                                                                                        \

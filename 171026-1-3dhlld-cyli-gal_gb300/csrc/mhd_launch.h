@@ -6,14 +6,10 @@
 #ifndef MHD_LAUNCH_H
 #define MHD_LAUNCH_H
 
-#include <cuda.h>   /* CUtensorMap (a type only: the library does not link the driver API) */
-
 #include "mhd_dev.cuh"
 
-/* cells per tile of the TMA-staged update, and the width of its windows that
- * start up to 3 cells before the tile (TMA rows start on 16-byte boundaries) */
+/* slots per tile of the update staged by bulk copies (a multiple of 32) */
 #define MHD_UPD_TILE 128
-#define MHD_UPD_WIDE 136
 
 namespace mhd {
 
@@ -25,15 +21,6 @@ struct Box {
 struct MaxLoc {
     double v;
     long long q;
-};
-
-/* Tensor maps of the arrays the TMA-staged update reads (precision form),
- * each array viewed as a 2D FP32 tensor [nvar][nc] with row stride nc */
-struct UpdMaps {
-    CUtensorMap v[2];          /* Va, Vb: box {MHD_UPD_TILE, 9} */
-    CUtensorMap f, g, un, u1;  /* F, G, U, U1: box {MHD_UPD_TILE, 9} */
-    CUtensorMap fm, gm, h;     /* F, G, H: box {MHD_UPD_WIDE, 9} */
-    CUtensorMap rho;           /* rhofloor: box {MHD_UPD_TILE, 1} */
 };
 
 template <typename T>
@@ -65,8 +52,10 @@ struct PairArgs {
 
 cudaError_t launch_update_pair(const Geom &G, const StageArgs<float> &a, const PairArgs &p, cudaStream_t st);
 cudaError_t launch_ghost_pair(const Geom &G, const StageArgs<float> &a, const PairArgs &p, cudaStream_t st);
-cudaError_t launch_cvt_pair(const double *src, float *hi, float *lo, long long n, cudaStream_t st);
-cudaError_t launch_cvt_pair_back(const float *hi, const float *lo, double *dst, long long n, cudaStream_t st);
+cudaError_t launch_cvt_pair(const Geom &G, const double *src, float *hi, float *lo, long long off, long long n,
+                            cudaStream_t st);
+cudaError_t launch_cvt_pair_back(const Geom &G, const float *hi, const float *lo, double *dst, long long off,
+                                 long long n, cudaStream_t st);
 cudaError_t launch_derive_v_pair(const Geom &G, const float *U, const float *Ulo, float *V, cudaStream_t st);
 
 #define MHD_DECLARE_LAUNCHERS(T)                                                                             \
@@ -83,8 +72,8 @@ cudaError_t launch_derive_v_pair(const Geom &G, const float *U, const float *Ulo
     cudaError_t launch_flux_zlast(const Geom &G, const T *Vinit, const StepScalars *sc, T *H, T *Hb,        \
                                   const T *Zs, int Hfull, cudaStream_t st); /* ... face kzmax-2 */          \
     cudaError_t launch_update(const Geom &G, const StageArgs<T> &a, cudaStream_t st);                        \
-    cudaError_t launch_update_tma(const Geom &G, const StageArgs<T> &a, const UpdMaps &maps, int vpar,      \
-                                  int *err, cudaStream_t st); /* precision form only */                    \
+    cudaError_t launch_update_tma(const Geom &G, const StageArgs<T> &a, int *err,                            \
+                                  cudaStream_t st); /* precision form only */                                \
     cudaError_t launch_ghost(const Geom &G, const StageArgs<T> &a, cudaStream_t st);                         \
     cudaError_t launch_stage(const Geom &G, const StageArgs<T> &a, int tj, int seg, cudaStream_t st);        \
     cudaError_t prepare_stage(T *); /* shared-memory attribute of the fused kernels */                       \
@@ -92,8 +81,12 @@ cudaError_t launch_derive_v_pair(const Geom &G, const float *U, const float *Ulo
     cudaError_t launch_setdt(const Geom &G, const T *V, MaxLoc *part, int nblk, cudaStream_t st);            \
     cudaError_t launch_source(const Geom &G, const T *V, const StepScalars *sc, const double *trig,          \
                               const float *trigf, double *S, cudaStream_t st);                               \
-    cudaError_t launch_cvt(const double *src, T *dst, long long n, cudaStream_t st);                         \
-    cudaError_t launch_cvt_back(const T *src, double *dst, long long n, cudaStream_t st);                    \
+    /* host-layout values off .. off+n-1 of an array of nvar variables (9, or 1) into / out of a state array;  \
+     * nvar = 0: out of a plain array */                                                                     \
+    cudaError_t launch_cvt(const Geom &G, int nvar, const double *src, T *dst, long long off, long long n,   \
+                           cudaStream_t st);                                                                 \
+    cudaError_t launch_cvt_back(const Geom &G, int nvar, const T *src, double *dst, long long off,           \
+                                long long n, cudaStream_t st);                                               \
     cudaError_t launch_derive_v(const Geom &G, const T *U, T *V, cudaStream_t st);
 
 MHD_DECLARE_LAUNCHERS(double)

@@ -121,7 +121,7 @@ __device__ __forceinline__ void absorb_pair(const Geom &G, const float *__restri
                                             bool zright, float uh[9], float ul[9])
 {
     const Tabs<double> &tb = G.d;
-    const long long q = cidx(G, i, j, k);
+    const float *ui0 = Uinit + slot0<float>(cidx<float>(G, i, j, k));
     const int ix0 = G.ixmax - 11, kz0 = G.kzmax - 11;
     const bool ax = i >= ix0, ac = i <= G.irin, az = zright && k >= kz0;
     if (!(ax || ac || az)) return;
@@ -129,7 +129,7 @@ __device__ __forceinline__ void absorb_pair(const Geom &G, const float *__restri
     const double fz = az ? tb.zabs[k - kz0] : 0.0;
 #pragma unroll
     for (int m = 0; m < 9; m++) {
-        const double ui = Uinit[m * G.nc + q];
+        const double ui = ui0[32 * m];
         double v = (double)uh[m] + (double)ul[m];
         if (ax) v -= (fx * (v - ui));
         if (ac) v -= (fc * (v - ui));
@@ -139,18 +139,17 @@ __device__ __forceinline__ void absorb_pair(const Geom &G, const float *__restri
     }
 }
 
-/* the stored pair state and primitives of one cell */
-__device__ __forceinline__ void store_pair(const Geom &G, const StageArgs<float> &a, const PairArgs &p, long long q,
+/* the stored pair state and primitives of one cell (b = slot0 of its slot) */
+__device__ __forceinline__ void store_pair(const StageArgs<float> &a, const PairArgs &p, long long b,
                                            const float uh[9], const float ul[9], const float W[9])
 {
-    const long long nc = G.nc;
     const bool to_u1 = a.kind == 0 || a.kind == 1;
     float *Uo = to_u1 ? a.U1 : a.Un, *Ul = to_u1 ? p.U1lo : p.Unlo;
 #pragma unroll
     for (int m = 0; m < 9; m++) {
-        Uo[m * nc + q] = uh[m];
-        Ul[m * nc + q] = ul[m];
-        a.Vout[m * nc + q] = W[m];
+        Uo[32 * m + b] = uh[m];
+        Ul[32 * m + b] = ul[m];
+        a.Vout[32 * m + b] = W[m];
     }
 }
 
@@ -170,7 +169,7 @@ __device__ __forceinline__ void zghost_fill_pair(const Geom &G, const StageArgs<
         else if (k == 1) kg = G.kzmax - 1;
         else return;
     }
-    const long long qg = cidx(G, i, j, kg);
+    const long long qg = cidx<float>(G, i, j, kg);
     float gh[9], gl[9], W[9];
 #pragma unroll
     for (int m = 0; m < 9; m++) {
@@ -180,7 +179,7 @@ __device__ __forceinline__ void zghost_fill_pair(const Geom &G, const StageArgs<
     }
     if (a.last) absorb_pair(G, a.Uinit, i, j, kg, G.scheme == MHD_SCHEME_RK2, gh, gl);
     const int flags = utov_check_pair(G, i, a.rhofloor[qg], gh, gl, W);
-    store_pair(G, a, p, qg, gh, gl, W);
+    store_pair(a, p, slot0<float>(qg), gh, gl, W);
     if (flags & 1) atomicAdd(&a.counters[0], 1);
     if (flags & 2) atomicAdd(&a.counters[1], 1);
     if (flags & 4) atomicAdd(&a.counters[2], 1);
@@ -195,8 +194,9 @@ __device__ __forceinline__ void zghost_fill_pair(const Geom &G, const StageArgs<
 __device__ __forceinline__ int update_cell_pair(const Geom &G, const StageArgs<float> &a, const PairArgs &p, int i,
                                                 int j, int k)
 {
-    const long long nc = G.nc, q = cidx(G, i, j, k);
-    const long long si = (long long)G.jymax * G.kzmax, sj = G.kzmax;
+    const long long q = cidx<float>(G, i, j, k), b = slot0<float>(q);
+    const long long bi = nslot<float, 0>(G, q, b, -1), bj = nslot<float, 1>(G, q, b, -1),
+                    bk = nslot<float, 2>(G, q, b, -1);
     const StepScalars *sc = a.sc;
     const float dt = sc->dtf;
     const int kind = a.kind;
@@ -206,8 +206,8 @@ __device__ __forceinline__ int update_cell_pair(const Geom &G, const StageArgs<f
     /* in three phases, as the FP32 update: the flux divergence (54 loads;
      * the last z face of a row from the compact Hb), the primitives and
      * sources, then the pair states and the combination */
-    const float *hu = a.H + q;
-    long long hs = nc;
+    const float *hu = a.H + b;
+    long long hs = 32;
     if (a.Hb && k == G.kzmax - 2) {
         hu = a.Hb + (long long)(i - 1) * (G.jymax - 2) + (j - 1);
         hs = (long long)(G.ixmax - 2) * (G.jymax - 2);
@@ -215,15 +215,15 @@ __device__ __forceinline__ int update_cell_pair(const Geom &G, const StageArgs<f
     geo_factors<float>(G, i, k, g);
 #pragma unroll
     for (int m = 0; m < 9; m++) {
-        const long long mq = m * nc + q;
-        div[m] = flux_div<float>(g, a.F[mq], a.F[mq - si], a.G[mq], a.G[mq - sj], hu[m * hs], a.H[mq - 1]);
+        const int mn = 32 * m;
+        div[m] = flux_div<float>(g, a.F[mn + b], a.F[mn + bi], a.G[mn + b], a.G[mn + bj], hu[m * hs], a.H[mn + bk]);
     }
 #pragma unroll
-    for (int m = 0; m < 9; m++) W[m] = a.V[m * nc + q];
+    for (int m = 0; m < 9; m++) W[m] = a.V[32 * m + b];
     source_at<float>(G, *sc, a.trig, a.trigf, i, j, k, W, S);
 #pragma unroll
     for (int m = 0; m < 9; m++) {
-        const long long mq = m * nc + q;
+        const long long mq = 32 * m + b;
         float unh = a.Un[mq], unl = p.Unlo[mq];
         float u1h = 0.0f, u1l = 0.0f;
         if (kind != 0) { u1h = a.U1[mq]; u1l = p.U1lo[mq]; }
@@ -241,13 +241,13 @@ __device__ __forceinline__ int update_cell_pair(const Geom &G, const StageArgs<f
     }
     if (is_bc_source(G, i, j, k)) {
 #pragma unroll
-        for (int m = 0; m < 9; m++) { a.Uraw[m * nc + q] = uh[m]; p.Urawlo[m * nc + q] = ul[m]; }
+        for (int m = 0; m < 9; m++) { a.Uraw[32 * m + b] = uh[m]; p.Urawlo[32 * m + b] = ul[m]; }
         if (a.zghost) zghost_fill_pair(G, a, p, i, j, k, uh, ul);
     }
     if (G.scheme == MHD_SCHEME_RK2 && k == 1) { uh[3] = 0.0f; ul[3] = 0.0f; }   /* zboundary.h:87 */
     if (a.last) absorb_pair(G, a.Uinit, i, j, k, G.scheme == MHD_SCHEME_RK2, uh, ul);
     const int flags = utov_check_pair(G, i, a.rhofloor[q], uh, ul, W);
-    store_pair(G, a, p, q, uh, ul, W);
+    store_pair(a, p, b, uh, ul, W);
     return flags;
 }
 
@@ -273,11 +273,11 @@ __global__ void __launch_bounds__(128) ghost_pair_kernel(Geom G, StageArgs<float
         unsigned neg;
         ghost_cell_of(G, tid, a.zghost, i, j, k);
         ghost_source(G, i, j, k, si, sj, sk, neg);
-        const long long nc = G.nc, q = cidx(G, i, j, k), qs = cidx(G, si, sj, sk);
+        const long long q = cidx<float>(G, i, j, k), bs = slot0<float>(cidx<float>(G, si, sj, sk));
         float uh[9], ul[9], W[9];
 #pragma unroll
         for (int m = 0; m < 9; m++) {
-            const float h = a.Uraw[m * nc + qs], l = p.Urawlo[m * nc + qs];
+            const float h = a.Uraw[32 * m + bs], l = p.Urawlo[32 * m + bs];
             const bool n = (neg >> m) & 1u;
             uh[m] = n ? -h : h;
             ul[m] = n ? -l : l;
@@ -285,43 +285,44 @@ __global__ void __launch_bounds__(128) ghost_pair_kernel(Geom G, StageArgs<float
         if (G.scheme == MHD_SCHEME_RK2 && k == 1) { uh[3] = 0.0f; ul[3] = 0.0f; }
         if (a.last) absorb_pair(G, a.Uinit, i, j, k, G.scheme == MHD_SCHEME_RK2, uh, ul);
         flags = utov_check_pair(G, i, a.rhofloor[q], uh, ul, W);
-        store_pair(G, a, p, q, uh, ul, W);
+        store_pair(a, p, slot0<float>(q), uh, ul, W);
     }
     add_counters(flags, a.counters);
 }
 
 /* FP64 host state -> pair (hi = the nearest FP32 value, lo = the rest) */
-__global__ void cvt_pair_from_f64(const double *__restrict__ src, float *__restrict__ hi, float *__restrict__ lo,
-                                  long long n)
+__global__ void cvt_pair_from_f64(Geom G, const double *__restrict__ src, float *__restrict__ hi,
+                                  float *__restrict__ lo, long long off, long long n)
 {
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const double v = src[t];
+    each_value<float>(G, 9, off, n, [&](long long s, long long d) {
+        const double v = src[s];
         const float h = (float)v;
-        hi[t] = h;
-        lo[t] = (float)(v - (double)h);
-    }
+        hi[d] = h;
+        lo[d] = (float)(v - (double)h);
+    });
 }
 
-__global__ void cvt_pair_to_f64(const float *__restrict__ hi, const float *__restrict__ lo, double *__restrict__ dst,
-                                long long n)
+__global__ void cvt_pair_to_f64(Geom G, const float *__restrict__ hi, const float *__restrict__ lo,
+                                double *__restrict__ dst, long long off, long long n)
 {
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
-        dst[t] = (double)hi[t] + (double)lo[t];
+    each_value<float>(G, 9, off, n, [&](long long s, long long d) { dst[s] = (double)hi[d] + (double)lo[d]; });
 }
 
 /* V = UtoV(U) of the pair state at every cell, ghosts included (no floors) */
 __global__ void __launch_bounds__(256) derive_v_pair_kernel(Geom G, const float *__restrict__ U,
                                                             const float *__restrict__ Ulo, float *__restrict__ V)
 {
-    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < G.nc;
-         q += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(q / ((long long)G.jymax * G.kzmax));
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < G.nc;
+         t += (long long)gridDim.x * blockDim.x) {
+        const long long r = t / G.kzmax;
+        const int i = (int)(r / G.jymax);
+        const long long b = slot0<float>(cidx<float>(G, i, (int)(r % G.jymax), (int)(t % G.kzmax)));
         float uh[9], ul[9], w[9];
 #pragma unroll
-        for (int m = 0; m < 9; m++) { uh[m] = U[m * G.nc + q]; ul[m] = Ulo[m * G.nc + q]; }
+        for (int m = 0; m < 9; m++) { uh[m] = U[32 * m + b]; ul[m] = Ulo[32 * m + b]; }
         utov_pair(G, i, uh, ul, w);
 #pragma unroll
-        for (int m = 0; m < 9; m++) V[m * G.nc + q] = w[m];
+        for (int m = 0; m < 9; m++) V[32 * m + b] = w[m];
     }
 }
 
@@ -346,15 +347,16 @@ __global__ void __launch_bounds__(256) derive_v_pair_kernel(Geom G, const float 
         ghost_pair_kernel<<<nblocks(ng, 128), 128, 0, st>>>(G, a, p);                                        \
         return cudaGetLastError();                                                                           \
     }                                                                                                        \
-    cudaError_t launch_cvt_pair(const double *src, float *hi, float *lo, long long n, cudaStream_t st)       \
+    cudaError_t launch_cvt_pair(const Geom &G, const double *src, float *hi, float *lo, long long off,        \
+                                long long n, cudaStream_t st)                                                 \
     {                                                                                                        \
-        cvt_pair_from_f64<<<1024, 256, 0, st>>>(src, hi, lo, n);                                             \
+        cvt_pair_from_f64<<<1024, 256, 0, st>>>(G, src, hi, lo, off, n);                                        \
         return cudaGetLastError();                                                                           \
     }                                                                                                        \
-    cudaError_t launch_cvt_pair_back(const float *hi, const float *lo, double *dst, long long n,             \
-                                     cudaStream_t st)                                                        \
+    cudaError_t launch_cvt_pair_back(const Geom &G, const float *hi, const float *lo, double *dst,           \
+                                     long long off, long long n, cudaStream_t st)                            \
     {                                                                                                        \
-        cvt_pair_to_f64<<<1024, 256, 0, st>>>(hi, lo, dst, n);                                               \
+        cvt_pair_to_f64<<<1024, 256, 0, st>>>(G, hi, lo, dst, off, n);                                          \
         return cudaGetLastError();                                                                           \
     }                                                                                                        \
     cudaError_t launch_derive_v_pair(const Geom &G, const float *U, const float *Ulo, float *V,              \

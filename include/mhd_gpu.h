@@ -271,7 +271,7 @@ int mhd_prof_read(mhd_ctx *ctx, double ms[MHD_PROF_NKIND], long long launches[MH
 int mhd_set_stage_shape(mhd_ctx *ctx, int fused, int tj, int seg);
 /* How the split stage's update reads its inputs (precision form): tma = 0
  * (the default) loads them thread by thread; tma = 1 stages each tile of 128
- * cells in shared memory with tensor copies, where the layout allows it
+ * cells in shared memory with bulk copies, where the grid allows it
  * (cells per variable a multiple of 4).  MHD_ERR_ARG for tma = 1 where it is
  * not available (plain form, other layouts); tma = 2 (precision form) keeps
  * the thread loads and has each block prefetch the streamed inputs of the
