@@ -1111,9 +1111,9 @@ __device__ __forceinline__ double cfl_rate64(const Geom &G, const T *__restrict_
     double v4 = v[4 * nc], v5 = v[5 * nc], v6 = v[6 * nc], v7 = v[7 * nc];
     double v2 = v1 * v1 + v2v * v2v + v3 * v3;
     double b2 = v4 * v4 + v5 * v5 + v6 * v6;
-    double t1 = sqrt(v2 + (MHD_GM * v7 + b2) / v0) / G.minlength[(long long)i * G.kzmax + k];
+    double t1 = x_div(x_sqrt(v2 + x_div(MHD_GM * v7 + b2, v0)), G.minlength[(long long)i * G.kzmax + k]);
     int cl = G.cooling ? cooling_rate(v0, v7) : 0;
-    double tc = (2.0 * ((v0 * v0 * cl) / (1.5 * v7)));
+    double tc = (2.0 * x_div(v0 * v0 * cl, 1.5 * v7));
     return rmax<double>(t1, tc);
 }
 
@@ -1132,9 +1132,9 @@ __device__ __forceinline__ double cfl_rate64_strict(const Geom &G, const T *__re
     double v4 = v[4 * nc], v5 = v[5 * nc], v6 = v[6 * nc], v7 = v[7 * nc];
     double v2 = v1 * v1 + v2v * v2v + v3 * v3;
     double b2 = v4 * v4 + v5 * v5 + v6 * v6;
-    double t1 = sqrt(v2 + (MHD_GM * v7 + b2) / v0) / G.minlength[(long long)i * G.kzmax + k];
+    double t1 = x_div(x_sqrt(v2 + x_div(MHD_GM * v7 + b2, v0)), G.minlength[(long long)i * G.kzmax + k]);
     int cl = G.cooling ? cooling_rate(v0, v7) : 0;
-    double tc = (2.0 * ((v0 * v0 * cl) / (1.5 * v7)));
+    double tc = (2.0 * x_div(v0 * v0 * cl, 1.5 * v7));
     if (t1 != t1 || tc != tc) return INFINITY;
     return rmax<double>(t1, tc);
 }
