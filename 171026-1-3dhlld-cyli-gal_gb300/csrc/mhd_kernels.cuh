@@ -30,6 +30,11 @@
 #define MHD_MARCH_RUN 16
 #endif
 
+/* the plain form's flux kernels: resident blocks of 128 threads (128 registers).
+ * At 256x256x128, MC: r 4.83 ms, phi 2.67 (3.32 with the registers it takes
+ * unbounded), z 4.77 (4.85); 5 blocks spill (5.02, 2.67, 5.19). */
+#define MHD_F64_MINB 4
+
 namespace mhd {
 
 /* ------------------------------------------------------------------------ */
@@ -128,7 +133,7 @@ __device__ __forceinline__ void march_run(const Geom &G, const T *__restrict__ V
  * the run, so the edge faces never diverge inside a warp.  Same operations
  * per state as face_states, so the plain form keeps its bits. */
 template <typename T, int DIR, int MR, bool REFLAYOUT>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, sizeof(T) == 8 ? MHD_F64_MINB : 1)
 march_flux_kernel(Geom G, const T *__restrict__ V, const T *__restrict__ Vinit, const StepScalars *__restrict__ sc,
                   T *__restrict__ F, Box b)
 {
@@ -229,7 +234,7 @@ zwalk_flux_kernel(Geom G, const T *__restrict__ V, const StepScalars *__restrict
  * The states are the values face_states forms (cell_slots equals recon_slot
  * bit for bit), so the plain form keeps its bits. */
 template <typename T>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 1)
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : MHD_F64_MINB)
 zwalk_edges_kernel(Geom G, const T *__restrict__ V, const T *__restrict__ Vinit, const StepScalars *__restrict__ sc,
                    T *__restrict__ F, T *__restrict__ Zs, Box b)
 {

@@ -30,7 +30,11 @@
 
 #ifdef __CUDACC__
 #define MHD_X64_FN __host__ __device__ __forceinline__
+/* division and root are called, not inlined: 24 copies a face do not fit the
+ * instruction cache (stalls for want of an instruction 3.3 -> 0.2 per issue) */
+#define MHD_X64_CALL static __host__ __device__ __noinline__
 #else
+#define MHD_X64_CALL static
 #define MHD_X64_FN static inline
 #endif
 
@@ -57,6 +61,12 @@ MHD_X64_FN float x_rcp(float f) { return 1.0f / f; }
 MHD_X64_FN float x_rsqrt(float f) { return 1.0f / sqrtf(f); }
 #endif
 
+/* a is an infinity or NaN */
+MHD_X64_FN bool x_special(double a) { return (x_hi(a) & 0x7ff00000u) == 0x7ff00000u; }
+MHD_X64_FN bool x_zero(double a) { return ((x_hi(a) << 1) | x_lo(a)) == 0u; }
+/* the magnitude's bits, ordered as the magnitude */
+MHD_X64_FN uint64_t x_mag(double a) { return (uint64_t)(x_hi(a) & 0x7fffffffu) << 32 | x_lo(a); }
+
 /* y in [0.5, 1] less 3 2^-23 as a fraction of 2^32: below the number that y,
  * off by 2^-22 at most, approximates */
 MHD_X64_FN uint32_t x_frac(float y)
@@ -65,7 +75,7 @@ MHD_X64_FN uint32_t x_frac(float y)
 }
 
 /* a / b */
-MHD_X64_FN double x_div(double a, double b)
+MHD_X64_CALL double x_div(double a, double b)
 {
     const uint32_t ah = x_hi(a), bh = x_hi(b), sign = (ah ^ bh) & 0x80000000u;
     const uint32_t ea = ah >> 20 & 0x7ffu, eb = bh >> 20 & 0x7ffu, er = ea - eb + 1023u;
@@ -94,7 +104,7 @@ MHD_X64_FN double x_div(double a, double b)
 }
 
 /* sqrt(a) */
-MHD_X64_FN double x_sqrt(double a)
+MHD_X64_CALL double x_sqrt(double a)
 {
     const uint32_t ah = x_hi(a), ea = ah >> 20;   /* with the sign: above 0x7ff for a negative */
     if (ea - 1u < 2046u) {
@@ -121,12 +131,6 @@ MHD_X64_FN double x_sqrt(double a)
     }
     return sqrt(a);
 }
-
-/* a is an infinity or NaN */
-MHD_X64_FN bool x_special(double a) { return (x_hi(a) & 0x7ff00000u) == 0x7ff00000u; }
-MHD_X64_FN bool x_zero(double a) { return ((x_hi(a) << 1) | x_lo(a)) == 0u; }
-/* the magnitude's bits, ordered as the magnitude */
-MHD_X64_FN uint64_t x_mag(double a) { return (uint64_t)(x_hi(a) & 0x7fffffffu) << 32 | x_lo(a); }
 
 /* a > b, a >= 0 and a <= 0 */
 MHD_X64_FN bool x_gt(double a, double b)
@@ -171,6 +175,31 @@ MHD_X64_FN double x_sign(double a)
 {
     if (x_special(a) || x_zero(a)) return fabs(a) / a;
     return x_of(x_hi(a) & 0x80000000u | 0x3ff00000u, 0u);
+}
+
+/* a times s, s the sign of x_sign */
+MHD_X64_FN double x_mulsign(double a, double s)
+{
+    if ((x_hi(s) & 0x7fffffffu) == 0x3ff00000u && x_lo(s) == 0u) return x_of(x_hi(a) ^ (x_hi(s) & 0x80000000u), x_lo(a));
+    return a * s;
+}
+/* (a + a s) / 2, s the sign of x_sign */
+MHD_X64_FN double x_doubled_half(double a, double s)
+{
+    if ((x_hi(a) >> 20 & 0x7ffu) < 2046u && (x_hi(s) & 0x7fffffffu) == 0x3ff00000u && x_lo(s) == 0u)
+        return (int32_t)x_hi(s) < 0 ? 0.0 : a;
+    return (a + a * s) * 0.5;
+}
+/* a 2^-1 and a 2^n (n = 1, 2) */
+MHD_X64_FN double x_half(double a)
+{
+    if ((x_hi(a) >> 20 & 0x7ffu) - 2u < 2045u) return x_of(x_hi(a) - 0x100000u, x_lo(a));
+    return x_zero(a) ? a : a * 0.5;
+}
+MHD_X64_FN double x_up(double a, int n)
+{
+    if ((x_hi(a) >> 20 & 0x7ffu) - 1u < 2043u) return x_of(x_hi(a) + ((uint32_t)n << 20), x_lo(a));
+    return x_zero(a) ? a : a * (double)(1 << n);
 }
 
 } /* namespace mhd */

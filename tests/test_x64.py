@@ -32,6 +32,14 @@ static void check(double a, double b, double c)
     same("ge0", x_ge0(a), a >= 0.0, a, b);
     same("le0", x_le0(a), a <= 0.0, a, b);
     same("sign", x_sign(a), fabs(a) / a, a, b);
+    const double one = B(b) >> 63 ? -1.0 : 1.0;
+    same("mulsign", x_mulsign(a, one), a * one, a, one);
+    same("mulsign", x_mulsign(a, b), a * b, a, b);
+    same("doubled_half", x_doubled_half(a, one), (a + a * one) * 0.5, a, one);
+    same("doubled_half", x_doubled_half(a, b), (a + a * b) * 0.5, a, b);
+    same("half", x_half(a), a * 0.5, a, b);
+    same("up", x_up(a, 1), a * 2.0, a, b);
+    same("up", x_up(a, 2), a * 4.0, a, b);
     same("minmod", x_same_sign(a, b) ? x_nearer(a, b) : 0.0,
          a * b <= 0.0 ? 0.0 : a > 0.0 ? rmin(a, b) : rmax(a, b), a, b);
     c = 0.25 * (a + b);
