@@ -32,7 +32,9 @@
 
 /* the plain form's flux kernels: resident blocks of 128 threads (128 registers).
  * At 256x256x128, MC: r 4.83 ms, phi 2.67 (3.32 with the registers it takes
- * unbounded), z 4.77 (4.85); 5 blocks spill (5.02, 2.67, 5.19). */
+ * unbounded), z 4.77 (4.85); 5 blocks spill (5.02, 2.67, 5.19).
+ * The FP32 marches have no bound (0, not 1: 64 registers against 90, a step of
+ * 512x512x256 19.1 ms against 20.0). */
 #define MHD_F64_MINB 4
 
 namespace mhd {
@@ -133,7 +135,7 @@ __device__ __forceinline__ void march_run(const Geom &G, const T *__restrict__ V
  * the run, so the edge faces never diverge inside a warp.  Same operations
  * per state as face_states, so the plain form keeps its bits. */
 template <typename T, int DIR, int MR, bool REFLAYOUT>
-__global__ void __launch_bounds__(128, sizeof(T) == 8 ? MHD_F64_MINB : 1)
+__global__ void __launch_bounds__(128, sizeof(T) == 8 ? MHD_F64_MINB : 0)
 march_flux_kernel(Geom G, const T *__restrict__ V, const T *__restrict__ Vinit, const StepScalars *__restrict__ sc,
                   T *__restrict__ F, Box b)
 {
