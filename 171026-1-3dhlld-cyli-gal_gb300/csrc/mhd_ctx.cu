@@ -661,10 +661,17 @@ static Box flux_box(const mhd_ctx *ctx, int dir)
 /* The split stage's face fluxes: r, phi, then the z row walk (every z face
  * but the last of each row, whose slots it leaves in the scratch Zs) and the
  * last z face of each row into the compact Hb -- and into H as well when the
- * TMA-staged update, which reads H directly, is selected (Hfull). */
+ * staged update, which reads H directly, is selected (Hfull).  One launch for
+ * all but the last z faces; one each while launches are timed. */
 template <typename T>
 static int split_fluxes(mhd_ctx *ctx, const T *V, const T *Vinit, T *F, T *Gf, T *H, int Hfull)
 {
+    if (!ctx->prof) {
+        CK(launch_flux3(ctx->G, V, Vinit, ctx->d_sc, F, Gf, H, (T *)ctx->Zs, ctx->st));
+        CK(launch_flux_zlast(ctx->G, Vinit, ctx->d_sc, H, (T *)ctx->Hb, (const T *)ctx->Zs, Hfull, ctx->st));
+        ctx->launches += 2;
+        return MHD_OK;
+    }
     LAUNCH(PK_FLUX_R, launch_flux(0, ctx->G, V, Vinit, ctx->d_sc, F, flux_box(ctx, 0), false, ctx->st));
     LAUNCH(PK_FLUX_PHI, launch_flux(1, ctx->G, V, Vinit, ctx->d_sc, Gf, flux_box(ctx, 1), false, ctx->st));
     /* one profiling slot for both z launches: every z face */

@@ -236,17 +236,12 @@ zwalk_flux_kernel(Geom G, const T *__restrict__ V, const StepScalars *__restrict
  * The states are the values face_states forms (cell_slots equals recon_slot
  * bit for bit), so the plain form keeps its bits. */
 template <typename T>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : MHD_F64_MINB)
-zwalk_edges_kernel(Geom G, const T *__restrict__ V, const T *__restrict__ Vinit, const StepScalars *__restrict__ sc,
-                   T *__restrict__ F, T *__restrict__ Zs, Box b)
+__device__ __forceinline__ void zwalk_edges_row(const Geom &G, const T *__restrict__ V, const T *__restrict__ Vinit,
+                                                const StepScalars *__restrict__ sc, T *__restrict__ F,
+                                                T *__restrict__ Zs, long long nrow, long long row)
 {
-    /* b: the interior rows i in [1, ixmax-1), j in [1, jymax-1) (indexing
-     * through the box keeps this kernel within 64 registers) */
-    const int nj = b.j1 - b.j0;
-    const long long nrow = (long long)(b.i1 - b.i0) * nj;
-    const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (row >= nrow) return;   /* a whole warp */
-    const int i = b.i0 + (int)(row / nj), j = b.j0 + (int)(row % nj);
+    const int nj = G.jymax - 2;
+    const int i = 1 + (int)(row / nj), j = 1 + (int)(row % nj);
     const int lane = threadIdx.x & 31;
     const int klast = G.kzmax - 2, lim = G.limiter;
     const T dt = Scal<T>::dt(sc), ch = Scal<T>::ch(sc), psicoef = Scal<T>::psi(sc);
@@ -301,11 +296,66 @@ zwalk_edges_kernel(Geom G, const T *__restrict__ V, const T *__restrict__ Vinit,
             store_face<T, false>(G, F, i, j, c - 1, Fo);
         }
     }
-    if (lane == 0) {   /* the left slot of cell kzmax-2 (the row index recomputed, not held) */
-        T *zr = Zs + ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
+    if (lane == 0) {   /* the left slot of cell kzmax-2 */
+        T *zr = Zs + row;
 #pragma unroll
         for (int m = 0; m < 9; m++) zr[m * nrow] = carry[m];
     }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : MHD_F64_MINB)
+zwalk_edges_kernel(Geom G, const T *__restrict__ V, const T *__restrict__ Vinit, const StepScalars *__restrict__ sc,
+                   T *__restrict__ F, T *__restrict__ Zs)
+{
+    const long long nrow = (long long)(G.ixmax - 2) * (G.jymax - 2);
+    const long long row = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (row >= nrow) return;   /* a whole warp */
+    zwalk_edges_row<T>(G, V, Vinit, sc, F, Zs, nrow, row);
+}
+
+/* The marched r or phi faces in blocks of 128 threads: mr faces per run, bx
+ * threads along k by 128 / bx lines, gx x gy blocks per run */
+struct MarchPlan {
+    int mr, bx, gx, gy, nblk;
+};
+
+/* All faces of the split stage but the last z face of each row in one launch:
+ * blocks of the r march, then of the phi march, then of the z walk, which only
+ * read V and write an array each.  Three launches one after another each wait
+ * for the last blocks of the one before, and on small grids none of them fills
+ * the GPU.  A step in FP32, three launches / one: 64x64x32 127 / 106 us,
+ * 128x128x64 465 / 456, 256x256x128 2664 / 2628, 512x512x256 19.09 / 19.20 ms;
+ * MC at 151x90x77 524 / 529, at 256x256x128 2743 / 2690.  The z walk's blocks are
+ * the shorter ones: taken first, 64x64x32 takes 110 us.  Bound by issue at 7
+ * resident blocks (72 registers); 8 blocks spill (2693 us at 256x256x128, z first),
+ * 6 hide less latency (2671 against 2638), and the three directions taken slab by
+ * slab along r, to share V in L2, gain 2 % there and lose 6 % at 64x64x32. */
+template <typename T>
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 7 : MHD_F64_MINB)
+flux3_kernel(Geom G, const T *__restrict__ V, const T *__restrict__ Vinit, const StepScalars *__restrict__ sc,
+             T *__restrict__ F, T *__restrict__ Gf, T *__restrict__ H, T *__restrict__ Zs, MarchPlan pr, MarchPlan pp)
+{
+    int b = blockIdx.x;
+    if (b < pr.nblk) {
+        const int k = 1 + (b % pr.gx) * pr.bx + threadIdx.x % pr.bx;
+        const int j = 1 + (b / pr.gx % pr.gy) * (128 / pr.bx) + threadIdx.x / pr.bx, f0 = b / (pr.gx * pr.gy) * pr.mr;
+        if (k < G.kzmax - 1 && j < G.jymax - 1)
+            march_run<T, 0, false>(G, V, Vinit, sc, F, j, k, f0, min(f0 + pr.mr, G.ixmax - 1));
+        return;
+    }
+    b -= pr.nblk;
+    if (b < pp.nblk) {
+        const int k = 1 + (b % pp.gx) * pp.bx + threadIdx.x % pp.bx;
+        const int i = 1 + (b / pp.gx % pp.gy) * (128 / pp.bx) + threadIdx.x / pp.bx, f0 = b / (pp.gx * pp.gy) * pp.mr;
+        if (k < G.kzmax - 1 && i < G.ixmax - 1)
+            march_run<T, 1, false>(G, V, Vinit, sc, Gf, i, k, f0, min(f0 + pp.mr, G.jymax - 1));
+        return;
+    }
+    b -= pp.nblk;
+    const long long nrow = (long long)(G.ixmax - 2) * (G.jymax - 2);
+    const long long row = (long long)b * 4 + (threadIdx.x >> 5);
+    if (row < nrow) zwalk_edges_row<T>(G, V, Vinit, sc, H, Zs, nrow, row);
 }
 
 /* The last z face (kzmax-2) of each (i,j) row from the slots
@@ -1350,9 +1400,7 @@ cudaError_t launch_flux_zwalk_t(const Geom &G, const T *V, const T *Vinit, const
     const long long nrow = (long long)(G.ixmax - 2) * (G.jymax - 2);
     if (G.kzmax < 4) return cudaErrorInvalidValue;
     if (nrow <= 0) return cudaSuccess;
-    Box b;
-    b.i0 = 1; b.i1 = G.ixmax - 1; b.j0 = 1; b.j1 = G.jymax - 1; b.k0 = 0; b.k1 = G.kzmax - 1;
-    zwalk_edges_kernel<T><<<nblocks(nrow, 4), 128, 0, st>>>(G, V, Vinit, sc, F, Zs, b);
+    zwalk_edges_kernel<T><<<nblocks(nrow, 4), 128, 0, st>>>(G, V, Vinit, sc, F, Zs);
     return cudaGetLastError();
 }
 
@@ -1365,6 +1413,42 @@ cudaError_t launch_flux_zlast_t(const Geom &G, const T *Vinit, const StepScalars
     const long long nrow = (long long)(G.ixmax - 2) * (G.jymax - 2);
     if (nrow <= 0) return cudaSuccess;
     zlast_flux_kernel<T><<<nblocks(nrow, 128), 128, 0, st>>>(G, Vinit, sc, H, Hb, Zs, Hfull);
+    return cudaGetLastError();
+}
+
+/* r / phi faces marched in runs along their direction: MHD_MARCH_RUN faces per
+ * thread where that still gives every SM several blocks, shorter runs on small
+ * grids (`lines` threads of nf faces) */
+static inline int march_length(long long lines, int nf)
+{
+    const long long want = 4LL * 128 * sm_count();
+    return lines * ((nf + MHD_MARCH_RUN - 1) / MHD_MARCH_RUN) >= want ? MHD_MARCH_RUN
+           : lines * ((nf + 3) / 4) >= want                          ? 4
+                                                                     : 1;
+}
+
+/* every z face but the last of each row, every r and phi face, in one launch */
+template <typename T>
+cudaError_t launch_flux3_t(const Geom &G, const T *V, const T *Vinit, const StepScalars *sc, T *F, T *Gf, T *H, T *Zs,
+                           cudaStream_t st)
+{
+    const int ni = G.ixmax - 2, nj = G.jymax - 2, nk = G.kzmax - 2;
+    const long long nrow = (long long)ni * nj;
+    if (G.kzmax < 4) return cudaErrorInvalidValue;
+    if (nrow <= 0) return cudaSuccess;
+    MarchPlan p[2];
+    for (int d = 0; d < 2; d++) {
+        const int nf = (d == 0 ? ni : nj) + 1, nl = d == 0 ? nj : ni;
+        dim3 gr, bl;
+        p[d].mr = march_length((long long)nk * nl, nf);
+        grid3(nk, nl, (nf + p[d].mr - 1) / p[d].mr, gr, bl);
+        p[d].bx = bl.x;
+        p[d].gx = gr.x;
+        p[d].gy = gr.y;
+        p[d].nblk = gr.x * gr.y * gr.z;
+    }
+    const unsigned nz = nblocks(nrow, 4);
+    flux3_kernel<T><<<nz + p[0].nblk + p[1].nblk, 128, 0, st>>>(G, V, Vinit, sc, F, Gf, H, Zs, p[0], p[1]);
     return cudaGetLastError();
 }
 
@@ -1388,14 +1472,9 @@ cudaError_t launch_flux_t(int dir, const Geom &G, const T *V, const T *Vinit, co
     }
     dim3 gr, bl;
     if (dir < 2) {
-        /* r / phi faces marched in runs along their direction: MHD_MARCH_RUN
-         * faces per thread where that still gives every SM several blocks,
-         * shorter runs on small grids */
         const int nf = dir == 0 ? b.i1 - b.i0 : b.j1 - b.j0;
         const long long lines = (long long)(b.k1 - b.k0) * (dir == 0 ? b.j1 - b.j0 : b.i1 - b.i0);
-        const long long want = 4LL * 128 * sm_count();
-        const int mr = reflayout || lines * ((nf + MHD_MARCH_RUN - 1) / MHD_MARCH_RUN) >= want ? MHD_MARCH_RUN
-                       : lines * ((nf + 3) / 4) >= want ? 4 : 1;
+        const int mr = reflayout ? MHD_MARCH_RUN : march_length(lines, nf);
         grid3(b.k1 - b.k0, dir == 0 ? b.j1 - b.j0 : b.i1 - b.i0, (nf + mr - 1) / mr, gr, bl);
 #define MHD_MARCH_CASE(D, MR, RL) march_flux_kernel<T, D, MR, RL><<<gr, bl, 0, st>>>(G, V, Vinit, sc, F, b)
         if (reflayout) {
@@ -1569,6 +1648,11 @@ cudaError_t launch_cvt_back_t(const Geom &G, int nvar, const T *src, double *dst
                                   T *Zs, cudaStream_t st)                                                    \
     {                                                                                                        \
         return launch_flux_zwalk_t<T>(G, V, Vinit, sc, F, Zs, st);                                           \
+    }                                                                                                        \
+    cudaError_t launch_flux3(const Geom &G, const T *V, const T *Vinit, const StepScalars *sc, T *F, T *Gf,  \
+                             T *H, T *Zs, cudaStream_t st)                                                   \
+    {                                                                                                        \
+        return launch_flux3_t<T>(G, V, Vinit, sc, F, Gf, H, Zs, st);                                         \
     }                                                                                                        \
     cudaError_t launch_flux_zlast(const Geom &G, const T *Vinit, const StepScalars *sc, T *H, T *Hb,        \
                                   const T *Zs, int Hfull, cudaStream_t st)                                   \

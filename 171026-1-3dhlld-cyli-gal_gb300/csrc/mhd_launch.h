@@ -69,6 +69,8 @@ cudaError_t launch_derive_v_pair(const Geom &G, const float *U, const float *Ulo
                              cudaStream_t st);                                                               \
     cudaError_t launch_flux_zwalk(const Geom &G, const T *V, const T *Vinit, const StepScalars *sc, T *F,    \
                                   T *Zs, cudaStream_t st); /* split stage: z faces 0 .. kzmax-3 */          \
+    cudaError_t launch_flux3(const Geom &G, const T *V, const T *Vinit, const StepScalars *sc, T *F, T *Gf,  \
+                             T *H, T *Zs, cudaStream_t st); /* r, phi and launch_flux_zwalk's z faces */     \
     cudaError_t launch_flux_zlast(const Geom &G, const T *Vinit, const StepScalars *sc, T *H, T *Hb,        \
                                   const T *Zs, int Hfull, cudaStream_t st); /* ... face kzmax-2 */          \
     cudaError_t launch_update(const Geom &G, const StageArgs<T> &a, cudaStream_t st);                        \
