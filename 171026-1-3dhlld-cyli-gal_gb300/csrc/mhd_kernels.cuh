@@ -24,6 +24,7 @@
 
 #include "mhd_dev.cuh"
 #include "mhd_launch.h"
+#include "mhd_march.h"
 
 /* faces per thread of the marched r and phi flux kernels */
 #ifndef MHD_MARCH_RUN
@@ -314,42 +315,31 @@ zwalk_edges_kernel(Geom G, const T *__restrict__ V, const T *__restrict__ Vinit,
     zwalk_edges_row<T>(G, V, Vinit, sc, F, Zs, nrow, row);
 }
 
-/* The marched r or phi faces in blocks of 128 threads: mr faces per run, bx
- * threads along k by 128 / bx lines, gx x gy blocks per run */
-struct MarchPlan {
-    int mr, bx, gx, gy, nblk;
-};
-
 /* All faces of the split stage but the last z face of each row in one launch:
- * blocks of the r march, then of the phi march, then of the z walk, which only
- * read V and write an array each.  Three launches one after another each wait
- * for the last blocks of the one before, and on small grids none of them fills
- * the GPU.  A step in FP32, three launches / one: 64x64x32 127 / 106 us,
- * 128x128x64 465 / 456, 256x256x128 2664 / 2628, 512x512x256 19.09 / 19.20 ms;
- * MC at 151x90x77 524 / 529, at 256x256x128 2743 / 2690.  The z walk's blocks are
- * the shorter ones: taken first, 64x64x32 takes 110 us.  Bound by issue at 7
- * resident blocks (72 registers); 8 blocks spill (2693 us at 256x256x128, z first),
- * 6 hide less latency (2671 against 2638), and the three directions taken slab by
- * slab along r, to share V in L2, gain 2 % there and lose 6 % at 64x64x32. */
+ * blocks of the r march, then of the phi march (which thread marches where:
+ * mhd_march.h), then of the z walk, which only read V and write an array each.
+ * Three launches one after another each wait for the last blocks of the one
+ * before, and on small grids none of them fills the GPU.  A step in FP32, three
+ * launches / one: 64x64x32 127 / 106 us, 128x128x64 465 / 456, 192x128x96 905 /
+ * 834, 256x256x128 2666 / 2625, 512x512x256 19.08 / 19.13 ms; MC at 151x90x77
+ * 516 / 492, at 256x256x128 2739 / 2683.  The z walk's blocks are the shorter
+ * ones: taken first, 64x64x32 takes 110 us.  Bound by issue at 7 resident blocks
+ * (72 registers); 8 blocks spill (2693 us at 256x256x128, z first), 6 hide less
+ * latency (2671 against 2638), and the three directions taken slab by slab along
+ * r, to share V in L2, gain 2 % there and lose 6 % at 64x64x32. */
 template <typename T>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 7 : MHD_F64_MINB)
 flux3_kernel(Geom G, const T *__restrict__ V, const T *__restrict__ Vinit, const StepScalars *__restrict__ sc,
              T *__restrict__ F, T *__restrict__ Gf, T *__restrict__ H, T *__restrict__ Zs, MarchPlan pr, MarchPlan pp)
 {
-    int b = blockIdx.x;
+    int b = blockIdx.x, line, k, f0, fe;
     if (b < pr.nblk) {
-        const int k = 1 + (b % pr.gx) * pr.bx + threadIdx.x % pr.bx;
-        const int j = 1 + (b / pr.gx % pr.gy) * (128 / pr.bx) + threadIdx.x / pr.bx, f0 = b / (pr.gx * pr.gy) * pr.mr;
-        if (k < G.kzmax - 1 && j < G.jymax - 1)
-            march_run<T, 0, false>(G, V, Vinit, sc, F, j, k, f0, min(f0 + pr.mr, G.ixmax - 1));
+        if (march_thread(pr, b, threadIdx.x, line, k, f0, fe)) march_run<T, 0, false>(G, V, Vinit, sc, F, line, k, f0, fe);
         return;
     }
     b -= pr.nblk;
     if (b < pp.nblk) {
-        const int k = 1 + (b % pp.gx) * pp.bx + threadIdx.x % pp.bx;
-        const int i = 1 + (b / pp.gx % pp.gy) * (128 / pp.bx) + threadIdx.x / pp.bx, f0 = b / (pp.gx * pp.gy) * pp.mr;
-        if (k < G.kzmax - 1 && i < G.ixmax - 1)
-            march_run<T, 1, false>(G, V, Vinit, sc, Gf, i, k, f0, min(f0 + pp.mr, G.jymax - 1));
+        if (march_thread(pp, b, threadIdx.x, line, k, f0, fe)) march_run<T, 1, false>(G, V, Vinit, sc, Gf, line, k, f0, fe);
         return;
     }
     b -= pp.nblk;
@@ -1448,13 +1438,7 @@ cudaError_t launch_flux3_t(const Geom &G, const T *V, const T *Vinit, const Step
     MarchPlan p[2];
     for (int d = 0; d < 2; d++) {
         const int nf = (d == 0 ? ni : nj) + 1, nl = d == 0 ? nj : ni;
-        dim3 gr, bl;
-        p[d].mr = march_length((long long)nk * nl, nf);
-        grid3(nk, nl, (nf + p[d].mr - 1) / p[d].mr, gr, bl);
-        p[d].bx = bl.x;
-        p[d].gx = gr.x;
-        p[d].gy = gr.y;
-        p[d].nblk = gr.x * gr.y * gr.z;
+        p[d] = march_plan(nk, nl, nf, march_length((long long)nk * nl, nf));
     }
     const unsigned nz = nblocks(nrow, 4);
     flux3_kernel<T><<<nz + p[0].nblk + p[1].nblk, 128, 0, st>>>(G, V, Vinit, sc, F, Gf, H, Zs, p[0], p[1]);
