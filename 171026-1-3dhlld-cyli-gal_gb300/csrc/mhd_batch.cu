@@ -324,8 +324,9 @@ batch_setdt_kernel(const DiscDev *__restrict__ discs, const uint2 *__restrict__ 
         for (int k = 1 + threadIdx.x; k < G.kzmax - 1; k += blockDim.x) {
             const long long q = cidx<float>(G, i, j, k);
             const float *v = V + slot0<float>(q);
-            float v0 = v[0], v1 = v[32], v2v = v[2 * 32], v3 = v[3 * 32];
-            float v4 = v[4 * 32], v5 = v[5 * 32], v6 = v[6 * 32], v7 = v[7 * 32];
+            constexpr int g = MHD_GROUP;
+            float v0 = v[0], v1 = v[g], v2v = v[2 * g], v3 = v[3 * g];
+            float v4 = v[4 * g], v5 = v[5 * g], v6 = v[6 * g], v7 = v[7 * g];
             float v2 = v1 * v1 + v2v * v2v + v3 * v3;
             float b2 = v4 * v4 + v5 * v5 + v6 * v6;
             float t1 = sqrtf(v2 + ((float)MHD_GM * v7 + b2) / v0) / G.f.minlength[(long long)i * G.kzmax + k];

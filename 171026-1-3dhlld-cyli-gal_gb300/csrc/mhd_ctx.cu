@@ -9,8 +9,8 @@
  *
  * Device data layout: in the plain form the reference's own, [m][i][j][k]
  * with k fastest and one ghost cell per side, so host<->device copies are plain
- * memcpy; the FP32 forms keep padded rows with the nine variables of 32 cells
- * together (cidx and slot0 in mhd_dev.cuh), written and read by the FP64
+ * memcpy; the FP32 forms keep padded rows in groups of slots, a group's nine variables
+ * together (mhd_layout.h), written and read by the FP64
  * conversion that their transfers make anyway.  The j-independent grid tables (geometric factors, minimum cell length,
  * axisymmetric gravity) are stored once per (i,k).  Compiled with
  * --fmad=false (the gravity probe and the FP64 scalars must round as the
@@ -339,8 +339,8 @@ extern "C" int mhd_create(const mhd_grid *g, const mhd_params *p, mhd_ctx **out)
 
     Geom &G = ctx->G;
     G.ixmax = ixmax; G.jymax = jymax; G.kzmax = kzmax; G.jy = g->jy; G.irin = g->irin; G.nc = nc;
-    G.kp = ctx->fp32 ? (kzmax + 31) / 32 * 32 : kzmax;
-    G.ncp = ctx->ncp = ctx->fp32 ? 32 + (long long)ixmax * jymax * G.kp : nc;
+    G.kp = ctx->fp32 ? row_slots(kzmax) : kzmax;
+    G.ncp = ctx->ncp = ctx->fp32 ? array_slots((long long)ixmax * jymax, G.kp) : nc;
     double *D = ctx->dtab;
     float *Fd = ctx->ftab;
     G.d.x = D + o_x; G.d.xm = D + o_xm; G.d.oneox = D + o_ox; G.d.oneodx = D + o_odx; G.d.oneodz = D + o_odz;

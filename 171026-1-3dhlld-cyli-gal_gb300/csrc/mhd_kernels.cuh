@@ -636,8 +636,8 @@ __device__ __forceinline__ void update_prefetch_ahead(const Geom &G, const Stage
     const int k0 = 1 + bx * blockDim.x, i = a.ibeg + bz;
     if (k0 >= G.kzmax - 1) return;
     const long long n9 = 9 * G.ncp;
-    /* the rows' cells k0 .. in whole groups of 32 slots: one run per row and array */
-    const int kn = 32 * ((min((int)blockDim.x, G.kzmax - 1 - k0) + 31) / 32);
+    /* the rows' cells k0 .. in whole groups: one run per row and array */
+    const int kn = row_slots(min((int)blockDim.x, G.kzmax - 1 - k0));
     for (int t = lane; t < 7 * (int)blockDim.y; t += 32) {
         const int arr = t / blockDim.y;
         const int j = 1 + by * blockDim.y + t % blockDim.y;
@@ -675,7 +675,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 9 : 1) update_kernel(Geo
 /* ------------------------------------------------------------------------ */
 /* TMA-staged update (precision form)                                        */
 /* ------------------------------------------------------------------------ */
-/* One block per tile of MHD_UPD_TILE consecutive slots (four groups of 32).
+/* One block per tile of MHD_UPD_TILE consecutive slots.
  * One thread loads the tile's inputs into shared memory with bulk copies
  * (cp.async.bulk, completing on an mbarrier): V, F, G, U^n, U^(k) and the
  * floor at the tile, F one plane and G one row below it, and H from the group
@@ -704,7 +704,7 @@ struct UpdTile {
     alignas(128) float u1[9 * MHD_UPD_TILE];
     alignas(128) float fm[9 * MHD_UPD_TILE];
     alignas(128) float gm[9 * MHD_UPD_TILE];
-    alignas(128) float h[9 * (MHD_UPD_TILE + 32)];   /* from the group before the tile */
+    alignas(128) float h[9 * (MHD_UPD_TILE + MHD_GROUP)];   /* from the group before the tile */
     alignas(128) float rho[MHD_UPD_TILE];
     alignas(8) unsigned long long bar;
 };
@@ -713,9 +713,9 @@ struct UpdTile {
 struct TileCell {
     const UpdTile &s;
     int t, b;
-    __device__ __forceinline__ float v(int m) const { return s.v[m * 32 + b]; }
-    __device__ __forceinline__ float un(int m) const { return s.un[m * 32 + b]; }
-    __device__ __forceinline__ float u1(int m) const { return s.u1[m * 32 + b]; }
+    __device__ __forceinline__ float v(int m) const { return s.v[m * MHD_GROUP + b]; }
+    __device__ __forceinline__ float un(int m) const { return s.un[m * MHD_GROUP + b]; }
+    __device__ __forceinline__ float u1(int m) const { return s.u1[m * MHD_GROUP + b]; }
     __device__ __forceinline__ float rho() const { return s.rho[t]; }
 };
 
@@ -754,7 +754,7 @@ update_tma_kernel(Geom G, StageArgs<T> a, long long qbeg, int *err, int spin)
     __syncthreads();
     if (threadIdx.x == 0) {
         const unsigned tile = 9 * MHD_UPD_TILE * 4, rho = MHD_UPD_TILE * 4;
-        const unsigned bytes = (a.kind != 0 ? 7 : 6) * tile + tile + 9 * 32 * 4 + rho;
+        const unsigned bytes = (a.kind != 0 ? 7 : 6) * tile + tile + 9 * MHD_GROUP * 4 + rho;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
                      :: "r"(smem_addr(&s.bar)), "r"(bytes) : "memory");
         bulk_load(s.v, a.V + b0, tile, &s.bar);
@@ -764,7 +764,7 @@ update_tma_kernel(Geom G, StageArgs<T> a, long long qbeg, int *err, int spin)
         if (a.kind != 0) bulk_load(s.u1, a.U1 + b0, tile, &s.bar);
         bulk_load(s.fm, a.F + nslot<T, 0>(G, q0, b0, -1), tile, &s.bar);
         bulk_load(s.gm, a.G + nslot<T, 1>(G, q0, b0, -1), tile, &s.bar);
-        bulk_load(s.h, a.H + b0 - 9 * 32, tile + 9 * 32 * 4, &s.bar);
+        bulk_load(s.h, a.H + b0 - 9 * MHD_GROUP, tile + 9 * MHD_GROUP * 4, &s.bar);
         bulk_load(s.rho, a.rhofloor + q0, rho, &s.bar);
     }
     bool ok = false;
@@ -779,13 +779,13 @@ update_tma_kernel(Geom G, StageArgs<T> a, long long qbeg, int *err, int spin)
     cell_of<T>(G, q, i, j, k);
     int flags = 0;
     if (i >= 1 && i <= G.ixmax - 2 && j >= 1 && j <= G.jymax - 2 && k >= 1 && k <= G.kzmax - 2) {
-        const int hu = b + 9 * 32, hl = (int)slot0<T>(t + 31);
+        const int hu = b + 9 * MHD_GROUP, hl = (int)slot0<T>(t + MHD_GROUP - 1);
         float gg[6], div[9];
         geo_factors<float>(G, i, k, gg);
 #pragma unroll
         for (int m = 0; m < 9; m++)
-            div[m] = flux_div<float>(gg, s.f[m * 32 + b], s.fm[m * 32 + b], s.g[m * 32 + b], s.gm[m * 32 + b],
-                                     s.h[m * 32 + hu], s.h[m * 32 + hl]);
+            div[m] = flux_div<float>(gg, s.f[m * MHD_GROUP + b], s.fm[m * MHD_GROUP + b], s.g[m * MHD_GROUP + b],
+                                     s.gm[m * MHD_GROUP + b], s.h[m * MHD_GROUP + hu], s.h[m * MHD_GROUP + hl]);
         flags = update_core<float>(G, a, i, j, k, q, div, TileCell{s, t, b});
     }
     add_counters(flags, a.counters);

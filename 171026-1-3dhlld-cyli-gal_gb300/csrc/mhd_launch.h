@@ -8,9 +8,6 @@
 
 #include "mhd_dev.cuh"
 
-/* slots per tile of the update staged by bulk copies (a multiple of 32) */
-#define MHD_UPD_TILE 128
-
 namespace mhd {
 
 /* half-open index box [i0,i1) x [j0,j1) x [k0,k1) */

@@ -129,7 +129,7 @@ __device__ __forceinline__ void absorb_pair(const Geom &G, const float *__restri
     const double fz = az ? tb.zabs[k - kz0] : 0.0;
 #pragma unroll
     for (int m = 0; m < 9; m++) {
-        const double ui = ui0[32 * m];
+        const double ui = ui0[MHD_GROUP * m];
         double v = (double)uh[m] + (double)ul[m];
         if (ax) v -= (fx * (v - ui));
         if (ac) v -= (fc * (v - ui));
@@ -147,9 +147,9 @@ __device__ __forceinline__ void store_pair(const StageArgs<float> &a, const Pair
     float *Uo = to_u1 ? a.U1 : a.Un, *Ul = to_u1 ? p.U1lo : p.Unlo;
 #pragma unroll
     for (int m = 0; m < 9; m++) {
-        Uo[32 * m + b] = uh[m];
-        Ul[32 * m + b] = ul[m];
-        a.Vout[32 * m + b] = W[m];
+        Uo[MHD_GROUP * m + b] = uh[m];
+        Ul[MHD_GROUP * m + b] = ul[m];
+        a.Vout[MHD_GROUP * m + b] = W[m];
     }
 }
 
@@ -207,7 +207,7 @@ __device__ __forceinline__ int update_cell_pair(const Geom &G, const StageArgs<f
      * the last z face of a row from the compact Hb), the primitives and
      * sources, then the pair states and the combination */
     const float *hu = a.H + b;
-    long long hs = 32;
+    long long hs = MHD_GROUP;
     if (a.Hb && k == G.kzmax - 2) {
         hu = a.Hb + (long long)(i - 1) * (G.jymax - 2) + (j - 1);
         hs = (long long)(G.ixmax - 2) * (G.jymax - 2);
@@ -215,15 +215,15 @@ __device__ __forceinline__ int update_cell_pair(const Geom &G, const StageArgs<f
     geo_factors<float>(G, i, k, g);
 #pragma unroll
     for (int m = 0; m < 9; m++) {
-        const int mn = 32 * m;
+        const int mn = MHD_GROUP * m;
         div[m] = flux_div<float>(g, a.F[mn + b], a.F[mn + bi], a.G[mn + b], a.G[mn + bj], hu[m * hs], a.H[mn + bk]);
     }
 #pragma unroll
-    for (int m = 0; m < 9; m++) W[m] = a.V[32 * m + b];
+    for (int m = 0; m < 9; m++) W[m] = a.V[MHD_GROUP * m + b];
     source_at<float>(G, *sc, a.trig, a.trigf, i, j, k, W, S);
 #pragma unroll
     for (int m = 0; m < 9; m++) {
-        const long long mq = 32 * m + b;
+        const long long mq = MHD_GROUP * m + b;
         float unh = a.Un[mq], unl = p.Unlo[mq];
         float u1h = 0.0f, u1l = 0.0f;
         if (kind != 0) { u1h = a.U1[mq]; u1l = p.U1lo[mq]; }
@@ -241,7 +241,7 @@ __device__ __forceinline__ int update_cell_pair(const Geom &G, const StageArgs<f
     }
     if (is_bc_source(G, i, j, k)) {
 #pragma unroll
-        for (int m = 0; m < 9; m++) { a.Uraw[32 * m + b] = uh[m]; p.Urawlo[32 * m + b] = ul[m]; }
+        for (int m = 0; m < 9; m++) { a.Uraw[MHD_GROUP * m + b] = uh[m]; p.Urawlo[MHD_GROUP * m + b] = ul[m]; }
         if (a.zghost) zghost_fill_pair(G, a, p, i, j, k, uh, ul);
     }
     if (G.scheme == MHD_SCHEME_RK2 && k == 1) { uh[3] = 0.0f; ul[3] = 0.0f; }   /* zboundary.h:87 */
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(128) ghost_pair_kernel(Geom G, StageArgs<float
         float uh[9], ul[9], W[9];
 #pragma unroll
         for (int m = 0; m < 9; m++) {
-            const float h = a.Uraw[32 * m + bs], l = p.Urawlo[32 * m + bs];
+            const float h = a.Uraw[MHD_GROUP * m + bs], l = p.Urawlo[MHD_GROUP * m + bs];
             const bool n = (neg >> m) & 1u;
             uh[m] = n ? -h : h;
             ul[m] = n ? -l : l;
@@ -319,10 +319,10 @@ __global__ void __launch_bounds__(256) derive_v_pair_kernel(Geom G, const float 
         const long long b = slot0<float>(cidx<float>(G, i, (int)(r % G.jymax), (int)(t % G.kzmax)));
         float uh[9], ul[9], w[9];
 #pragma unroll
-        for (int m = 0; m < 9; m++) { uh[m] = U[32 * m + b]; ul[m] = Ulo[32 * m + b]; }
+        for (int m = 0; m < 9; m++) { uh[m] = U[MHD_GROUP * m + b]; ul[m] = Ulo[MHD_GROUP * m + b]; }
         utov_pair(G, i, uh, ul, w);
 #pragma unroll
-        for (int m = 0; m < 9; m++) V[32 * m + b] = w[m];
+        for (int m = 0; m < 9; m++) V[MHD_GROUP * m + b] = w[m];
     }
 }
 
