@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "mhd_ctx_internal.h"
+#include "mhd_march.h"
 
 using namespace mhd;
 
@@ -662,11 +663,12 @@ static Box flux_box(const mhd_ctx *ctx, int dir)
  * but the last of each row, whose slots it leaves in the scratch Zs) and the
  * last z face of each row into the compact Hb -- and into H as well when the
  * staged update, which reads H directly, is selected (Hfull).  One launch for
- * all but the last z faces; one each while launches are timed. */
+ * all but the last z faces where one_face_launch says so; one each elsewhere and
+ * while launches are timed. */
 template <typename T>
 static int split_fluxes(mhd_ctx *ctx, const T *V, const T *Vinit, T *F, T *Gf, T *H, int Hfull)
 {
-    if (!ctx->prof) {
+    if (!ctx->prof && one_face_launch(ctx->fp32, ctx->p.limiter == MHD_LIMITER_SUPERBEE, ctx->ix, ctx->jy, ctx->kz)) {
         CK(launch_flux3(ctx->G, V, Vinit, ctx->d_sc, F, Gf, H, (T *)ctx->Zs, ctx->st));
         CK(launch_flux_zlast(ctx->G, Vinit, ctx->d_sc, H, (T *)ctx->Hb, (const T *)ctx->Zs, Hfull, ctx->st));
         ctx->launches += 2;

@@ -320,9 +320,9 @@ zwalk_edges_kernel(Geom G, const T *__restrict__ V, const T *__restrict__ Vinit,
  * mhd_march.h), then of the z walk, which only read V and write an array each.
  * Three launches one after another each wait for the last blocks of the one
  * before, and on small grids none of them fills the GPU.  A step in FP32, three
- * launches / one: 64x64x32 127 / 106 us, 128x128x64 465 / 456, 192x128x96 905 /
- * 834, 256x256x128 2666 / 2625, 512x512x256 19.08 / 19.13 ms; MC at 151x90x77
- * 516 / 492, at 256x256x128 2739 / 2683.  The z walk's blocks are the shorter
+ * launches / one: 64x64x32 127 / 106 us, 128x128x64 453 / 440, 192x128x96 905 /
+ * 834, 256x256x128 2663 / 2623; MC at 151x90x77 516 / 492; large grids:
+ * one_face_launch.  The z walk's blocks are the shorter
  * ones: taken first, 64x64x32 takes 110 us.  Bound by issue at 7 resident blocks
  * (72 registers); 8 blocks spill (2693 us at 256x256x128, z first), 6 hide less
  * latency (2671 against 2638), and the three directions taken slab by slab along

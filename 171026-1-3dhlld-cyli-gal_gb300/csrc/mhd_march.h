@@ -54,6 +54,33 @@ MHD_MARCH_FN bool march_thread(const MarchPlan &p, int b, int t, int &line, int 
     return w < p.warps && k <= p.nk;
 }
 
+/* Whether the r, phi and z faces of ni x nj x nk interior cells go into one
+ * launch, or into one per direction.  One launch fills the GPU where a
+ * direction alone does not, and packs rows of 5, 6, 7, 9 .. groups of 32 cells
+ * without idle warps, where a launch per direction takes rows in blocks of four
+ * warps (`whole`: it leaves none idle either).  On large FP32 grids the launches
+ * per direction win: their marches hold 62 to 64 registers instead of 72, and
+ * superbee, which waits on memory most, gains most.  A step in FP32, one launch
+ * / one per direction:
+ *   minmod   256x256x128 2623 / 2663 us, 384x384x256 10960 / 10964, 512x384x256
+ *            14567 / 14544, 512x512x256 19425 / 19360; rows of 7 groups:
+ *            512x512x224 17146 / 17237
+ *   van Leer 384x384x256 11244 / 11171, 512x512x256 19979 / 19721
+ *   superbee 192x160x128 2150 / 2243, 224x224x128 3455 / 3441, 384x384x128 9865 /
+ *            9387, 512x512x256 33643 / 31255; rows of 6 groups: 320x320x192
+ *            10172 / 10281, 512x256x192 12926 / 12823
+ * The pair-state form, the same faces, alike.  The plain form (128 registers
+ * either way): 512x512x192 324 / 327 ms. */
+static inline bool one_face_launch(bool fp32, bool superbee, int ni, int nj, int nk)
+{
+    const int groups = (nk + 31) / 32;
+    const bool whole = groups <= 4 || groups % 4 == 0;
+    const double cells = (double)ni * nj * nk;
+    if (!fp32) return true;
+    if (superbee) return cells < (whole ? 6e6 : 20e6);
+    return !whole || cells < 40e6;
+}
+
 } /* namespace mhd */
 
 #endif

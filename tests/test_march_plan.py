@@ -48,3 +48,30 @@ def test_each_face_has_one_thread(tmp_path):
     subprocess.check_call(["g++", "-std=c++17", "-O2", "-I", os.path.join(PKG, "csrc"), str(tmp_path / "t.cpp"), "-o", exe])
     r = subprocess.run([exe], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout
+
+
+RULE = r"""
+#include <cstdio>
+#include "mhd_march.h"
+int main()
+{
+    int fp32, superbee, ni, nj, nk;
+    while (scanf("%d %d %d %d %d", &fp32, &superbee, &ni, &nj, &nk) == 5) printf("%d\n", mhd::one_face_launch(fp32, superbee, ni, nj, nk));
+    return 0;
+}
+"""
+# FP32: cells on both sides of each line, in rows that a launch per direction
+# packs whole (1 to 4 groups of 32, or whole blocks of 4) and in rows that it
+# does not; the plain form always in one launch
+ONE = [(1, 0, 12, 4, 12), (1, 0, 384, 384, 256), (1, 0, 512, 512, 224), (1, 0, 640, 640, 160), (1, 1, 64, 64, 32),
+       (1, 1, 192, 160, 128), (1, 1, 320, 320, 192), (0, 0, 512, 512, 256), (0, 1, 512, 512, 256)]
+EACH = [(1, 0, 512, 384, 256), (1, 0, 512, 512, 250), (1, 0, 1024, 512, 128), (1, 1, 224, 224, 128), (1, 1, 384, 384, 64),
+        (1, 1, 512, 512, 96), (1, 1, 512, 256, 192), (1, 1, 512, 512, 256)]
+
+
+def test_which_grids_take_one_launch(tmp_path):
+    (tmp_path / "r.cpp").write_text(RULE)
+    exe = str(tmp_path / "r")
+    subprocess.check_call(["g++", "-std=c++17", "-O2", "-I", os.path.join(PKG, "csrc"), str(tmp_path / "r.cpp"), "-o", exe])
+    r = subprocess.run([exe], input="".join("%d %d %d %d %d\n" % c for c in ONE + EACH), capture_output=True, text=True)
+    assert r.stdout.split() == ["1"] * len(ONE) + ["0"] * len(EACH)
