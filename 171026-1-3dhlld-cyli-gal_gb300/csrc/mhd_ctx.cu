@@ -34,6 +34,9 @@ using namespace mhd;
 enum { PK_FLUX_R = 0, PK_FLUX_PHI = 1, PK_FLUX_Z = 2, PK_UPDATE = 3, PK_GHOST = 4, PK_SETDT = 5, PK_TRIG = 6,
        PK_CVT = 7, PK_STAGE = 8, PK_ZUPDATE = 9 };
 static const int MAXSLOT = 256;
+/* ctx->prof: launches not timed, timed as a step makes them, timed with the
+ * split stage's faces in a launch per direction */
+enum { PROF_OFF = 0, PROF_ON = 1, PROF_BY_DIRECTION = 2 };
 
 /* fold the recorded event pairs into the per-kind totals */
 static cudaError_t prof_harvest(mhd_ctx *ctx)
@@ -663,15 +666,18 @@ static Box flux_box(const mhd_ctx *ctx, int dir)
  * but the last of each row, whose slots it leaves in the scratch Zs) and the
  * last z face of each row into the compact Hb -- and into H as well when the
  * staged update, which reads H directly, is selected (Hfull).  One launch for
- * all but the last z faces where one_face_launch says so; one each elsewhere and
- * while launches are timed. */
+ * all but the last z faces where one_face_launch says so, timed with the last z
+ * faces as one; one each elsewhere, and where they are timed by direction. */
 template <typename T>
 static int split_fluxes(mhd_ctx *ctx, const T *V, const T *Vinit, T *F, T *Gf, T *H, int Hfull)
 {
-    if (!ctx->prof && one_face_launch(ctx->fp32, ctx->p.limiter == MHD_LIMITER_SUPERBEE, ctx->ix, ctx->jy, ctx->kz)) {
+    if (ctx->prof != PROF_BY_DIRECTION &&
+        one_face_launch(ctx->fp32, ctx->p.limiter == MHD_LIMITER_SUPERBEE, ctx->ix, ctx->jy, ctx->kz)) {
+        CK(prof_begin(ctx, PK_STAGE));
         CK(launch_flux3(ctx->G, V, Vinit, ctx->d_sc, F, Gf, H, (T *)ctx->Zs, ctx->st));
+        ctx->launches++;
         CK(launch_flux_zlast(ctx->G, Vinit, ctx->d_sc, H, (T *)ctx->Hb, (const T *)ctx->Zs, Hfull, ctx->st));
-        ctx->launches += 2;
+        CK(prof_end(ctx));
         return MHD_OK;
     }
     LAUNCH(PK_FLUX_R, launch_flux(0, ctx->G, V, Vinit, ctx->d_sc, F, flux_box(ctx, 0), false, ctx->st));
@@ -1220,7 +1226,7 @@ extern "C" int mhd_prof_enable(mhd_ctx *ctx, int on)
         for (int q = 0; q < 2 * MAXSLOT; q++) CK(cudaEventCreate(&ctx->ev[q]));
     ctx->nslot = 0;
     for (int k = 0; k < MHD_PROF_NKIND; k++) { ctx->prof_ms[k] = 0.0; ctx->prof_n[k] = 0; }
-    ctx->prof = on ? 1 : 0;
+    ctx->prof = on == 2 ? PROF_BY_DIRECTION : on ? PROF_ON : PROF_OFF;
     return MHD_OK;
 }
 

@@ -476,8 +476,11 @@ class Disc:
     PROF_KINDS = ["flux_r", "flux_phi", "flux_z", "update", "ghost", "setdt", "trig", "convert", "stage",
                   "zupdate"]
 
-    def prof(self, on=True):
-        check(lib().mhd_prof_enable(self.h, 1 if on else 0), "mhd_prof_enable")
+    def prof(self, on=True, by_direction=False):
+        """Time every launch (mhd_prof_enable); by_direction: the split stage's
+        faces in a launch per direction, else as the step makes them ("stage"
+        where they are one launch)."""
+        check(lib().mhd_prof_enable(self.h, (2 if by_direction else 1) if on else 0), "mhd_prof_enable")
 
     def prof_read(self):
         ms = np.zeros(len(self.PROF_KINDS))

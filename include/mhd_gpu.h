@@ -254,13 +254,17 @@ int mhd_checkpoint_wait(mhd_ctx *ctx);
 /* Per-kernel timing with CUDA events recorded around every launch on the
  * context's stream (off by default; enabling resets the totals).  Kinds:
  * 0 flux r, 1 flux phi, 2 flux z, 3 update, 4 ghost fill, 5 CFL reduction,
- * 6 arm-phase table, 7 state conversion, 8 fused stage (fluxes + update),
- * 9 z fluxes + update. */
+ * 6 arm-phase table, 7 state conversion, 8 phases joined in one launch (stage
+ * shape 0: the r, phi and z faces; shape 1: fluxes + update), 9 z fluxes +
+ * update.  on = 1 times the launches that the step makes anyway; on = 2 gives the
+ * faces of stage shape 0 a launch per direction on every grid (the same bits), so
+ * that kinds 0 to 2 are filled; 0 ends the timing. */
 #define MHD_PROF_NKIND 10
 int mhd_prof_enable(mhd_ctx *ctx, int on);
 int mhd_prof_read(mhd_ctx *ctx, double ms[MHD_PROF_NKIND], long long launches[MHD_PROF_NKIND]);
-/* How a stage runs.  fused = 0: three flux kernels write F, G, H to device
- * memory and an update kernel reads them; fused = 2: the r and phi flux
+/* How a stage runs.  fused = 0: the flux kernels (r, phi and z in one launch, or
+ * one each where that is faster) write F, G, H to device memory and an update
+ * kernel reads them; fused = 2: the r and phi flux
  * kernels, then one kernel forms the z fluxes in registers and updates the
  * cells; fused = 1: one kernel forms all fluxes on chip and updates the cells
  * (tile 32 k-cells x tj j-cells, tj = 7, marching over runs of seg cells in
