@@ -514,7 +514,8 @@ def kernel_bytes(dims, s, pair=False):
     """Algorithmic bytes per launch of each kernel: its unique inputs and
     outputs, s bytes per value (4 in the precision form, 8 in the plain form).
     A flux kernel reads each cell's 9 primitives once and writes 9 fluxes per
-    face (18 values per face); the update reads V, the three fluxes (27 values
+    face (18 values per face; "stage" is the three directions in one launch, which
+    large FP32 discs do not take); the update reads V, the three fluxes (27 values
     with their lower neighbours), U^n, U^(k) in two of the three RK3 stages and
     the density floor, and writes U and V (70 values per cell averaged over
     the stages); the CFL reduction reads 8 primitives of the cells of its
@@ -523,13 +524,14 @@ def kernel_bytes(dims, s, pair=False):
     100 by stage)."""
     nx, ny, nz = dims
     zones = nx * ny * nz
-    return {"flux_r": (nx + 1) * ny * nz * 18 * s,
-            "flux_phi": nx * (ny + 1) * nz * 18 * s,
-            "flux_z": nx * ny * (nz + 1) * 18 * s,      # every z face (the row walk and the last face of each row)
+    r, phi, z = (nx + 1) * ny * nz, nx * (ny + 1) * nz, nx * ny * (nz + 1)   # every face, the boundary ones too
+    return {"flux_r": r * 18 * s,
+            "flux_phi": phi * 18 * s,
+            "flux_z": z * 18 * s,
             "update": zones * (94 if pair else 70) * s,
             "setdt": (nx - 10) * ny * nz * 8 * s,
             "ghost": 0, "trig": 0, "convert": 0,
-            "stage": zones * (9 + 9 + 1 + 9 + 9 + 6) * s,
+            "stage": (r + phi + z) * 18 * s,
             "zupdate": zones * (70 - 9) * s}
 
 
@@ -694,10 +696,11 @@ def main():
     tot = sum(v[0] for v in kern.values())
     dom = max(kern, key=lambda k: kern[k][0])
     # DRAM bytes (read + write) per zone per launch from the ncu captures at
-    # 256x256x128 (profiles/), scaled here by the zones of this workload
+    # 256x256x128 (profiles/), scaled here by the zones of this workload; the
+    # update's in unpadded arrays (268 B per zone; in rows of whole groups of
+    # slots the same launch moves 277, of which 4 % are the rows' padding)
     measured_traffic = {"update": (1.613262e9 + 0.632994e9) / 8388608,
-                        "flux_r": (0.384357e9 + 0.262446e9) / 8388608,
-                        "flux_phi": (0.382199e9 + 0.262957e9) / 8388608}
+                        "stage": (1.066790e9 + 0.887214e9) / 8388608}
     traffic = measured_traffic[dom] * zones if dom in measured_traffic else None
     pk = per_kernel.get(dom, {})
     roof = {"bound": "hbm", "kernel": dom, "achieved": pk.get("gbs"), "peak": hbm_peak, "unit": "GB/s",
@@ -755,13 +758,15 @@ def main():
     d64.upload(U, V)
     if dist:
         dist.barrier()
-    ms64, wall64, l64, kern64, _ = time_steps(M, d64, f64_steps, 1, prof=True)
+    ms64, wall64, l64, _, _ = time_steps(M, d64, f64_steps, 1)
     ms64 = max_over_ranks(dist, ms64)
+    d64.upload(U, V)
+    _, _, _, kern64, _ = time_steps(M, d64, 2, 1, prof=True)
     v64 = zones * f64_steps * world / (ms64 / 1e3)
     fp64 = {"value": v64, "unit": "zone-updates/s", "steps": f64_steps, "ms_per_step": ms64 / f64_steps,
             "speedup_fp32_over_fp64": value / v64, "speedup_pair_over_fp64": pair["value"] / v64,
             "kernels": kernel_rooflines(kern64, kernel_bytes(dims, 8), hbm_peak),
-            "bound": "FP64 pipe: the flux kernels keep it 86 % active (ncu, profiles/flux_fp64_256x256x128.md); "
+            "bound": "FP64 pipe: the faces and the update keep it 84 % active (ncu, profiles/faces_256x256x128.md); "
                      "frac_hbm is each kernel's HBM fraction only"}
     link = None
     if not args.no_e2e:
