@@ -408,7 +408,8 @@ extern "C" int mhd_create(const mhd_grid *g, const mhd_params *p, mhd_ctx **out)
     CKC(cudaMallocHost((void **)&ctx->h_part, ctx->npart * sizeof(MaxLoc)));
     CKC(cudaMalloc((void **)&ctx->d_cnt, 3 * 3 * sizeof(int)));
     CKC(cudaMallocHost((void **)&ctx->h_cnt, 3 * 3 * sizeof(int)));
-    /* the sizes the staged update has always been offered for */
+    /* the sizes the staged update is offered for: those of the tensor maps that
+     * it once used.  The slots' layout would take any. */
     ctx->upd_bulk = ctx->fp32 && nc % 4 == 0 && nc + 2 * MHD_UPD_TILE < (1LL << 31);
     ctx->upd_tma = 0;
     ctx->stage_n = 1LL << 24;

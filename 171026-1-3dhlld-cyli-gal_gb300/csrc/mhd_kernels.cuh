@@ -688,14 +688,13 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 9 : 1) update_kernel(Geo
  * that second wait run out as well, the block exits while bulk copies may
  * still be writing its shared memory -- unsafe, which is one reason this path
  * is an option that stays off, and no test drives either wait to its limit.
- * Measured at 512x512x256 (with tensor copies of the [m][cells] layout): 3.62
- * ms per launch against 3.38 ms for update_kernel (3.69 ms with all on-chip
- * memory as shared memory): five
- * 38 KB tiles per SM keep more bytes in flight than the thread loads, but
+ * Measured at 512x512x256: 3.38 ms per launch against 3.33 ms for
+ * update_kernel, and the last z faces go to H as well (z faces 1.13 -> 1.18 ms):
+ * five 38 KB tiles per SM keep more bytes in flight than the thread loads, but
  * each block then computes with 4 warps and 20 per SM, and the update's
- * arithmetic (sources, the FP64 pressure repair) no longer hides under
- * other warps' loads.  An option (mhd_set_update_path); the thread loads stay
- * the default. */
+ * arithmetic (sources, the FP64 pressure repair) no longer hides under other
+ * warps' loads.  An option (mhd_set_update_path); the thread loads stay the
+ * default. */
 struct UpdTile {
     alignas(128) float v[9 * MHD_UPD_TILE];
     alignas(128) float f[9 * MHD_UPD_TILE];

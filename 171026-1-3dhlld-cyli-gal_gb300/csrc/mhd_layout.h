@@ -16,9 +16,9 @@
  * between a row's end and its neighbour's ghost.  A step in FP32, groups of 32
  * / 16 / 8: 256x256x12 802 / 688 / 683 us, 256x256x32 878 / 860 / 831,
  * 256x256x48 1381 / 1324 / 1296, 256x256x128 2624 / 2613 / 2615, 151x90x77 (MC)
- * 497 / 469 / 469, 64x64x32 109 / 106 / 105; 512x512x256 19.13 / 19.15 / 19.41
- * ms, where the rounding is small and four lines a load cost more than they
- * save.  The same bits throughout.
+ * 497 / 469 / 469, 64x64x32 109 / 106 / 105; 512x512x256 19.08 / 19.00 / 19.35
+ * ms (pair state 24.32 / 24.29 / 24.59), where the rounding is small and four
+ * lines a load cost more than they save.  The same bits throughout.
  *
  * Plain C++: the host compiles it too, for the tests.
  */

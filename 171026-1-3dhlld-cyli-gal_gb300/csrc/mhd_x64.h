@@ -2,11 +2,12 @@
  * mhd_x64.h -- IEEE double division, square root, comparisons and a minmod
  * slope on the 32-bit integer pipe, bit for bit what the FP64 unit gives.
  *
- * The plain form's kernels keep the FP64 pipe 86 % active: it has two lanes
- * per SM, so a warp instruction takes 16 cycles of it while the integer pipes
- * and the schedulers idle.  A division or a square root is eight or nine such
+ * The plain form's kernels are bound by the FP64 pipe: it has two lanes per SM,
+ * so a warp instruction takes 16 cycles of it while the integer pipes and the
+ * schedulers idle.  A division or a square root is eight or nine such
  * instructions; here it is about 75 integer ones, and leaves the pipe to the
- * additions and multiplications.
+ * additions and multiplications (the pipe stays 84 % active, with about 350 FP64
+ * instructions per r face where the compiler's division and root take 600).
  *
  * Division and square root are digit recurrences (Ercegovac and Lang, Division
  * and Square Root: Digit-Recurrence Algorithms and Implementations) of three

@@ -503,7 +503,7 @@ class Disc:
 
     def set_update_path(self, tma):
         """1: the split stage's update stages its tiles in shared memory with
-        tensor copies; 0: thread-by-thread loads (mhd_set_update_path)."""
+        bulk copies; 0: thread-by-thread loads (mhd_set_update_path)."""
         check(lib().mhd_set_update_path(self.h, int(tma)), "mhd_set_update_path")
 
     def set_state_rounding(self, on=True):
