@@ -42,11 +42,12 @@ static inline MarchPlan march_plan(int nk, int nl, int nf, int mr)
 }
 
 /* thread t (of 128) of block b: its line and cell, from 1, and its faces f0 ..
- * fe-1; false where it has none */
+ * fe-1; false where it has none.  Divided as unsigned: the signs' handling took
+ * registers that the plain form's faces do not have (20 words reloaded a face). */
 MHD_MARCH_FN bool march_thread(const MarchPlan &p, int b, int t, int &line, int &k, int &f0, int &fe)
 {
-    const int run = b / p.run_blocks, w = (b - run * p.run_blocks) * 4 + (t >> 5);
-    const int l = w / p.groups;
+    const int run = (int)((unsigned)b / (unsigned)p.run_blocks), w = (b - run * p.run_blocks) * 4 + (int)((unsigned)t >> 5);
+    const int l = (int)((unsigned)w / (unsigned)p.groups);
     line = 1 + l;
     k = 1 + (w - l * p.groups) * 32 + (t & 31);
     f0 = run * p.mr;
